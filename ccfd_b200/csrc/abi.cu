@@ -122,6 +122,8 @@ static void free_device(ccfd_ctx* ctx) {
     ccfd_implicit_free(ctx);
     for (void* p : ctx->allocs) cudaFreeAsync(p, ctx->stream);
     ctx->allocs.clear();
+    ctx->fstate = nullptr;
+    ctx->grad_f = nullptr;
     ctx->device_bytes = 0;
     ctx->uploaded = false;
 }
@@ -186,10 +188,6 @@ extern "C" int ccfd_create(const ccfd_params* params, ccfd_ctx** out) {
         for (int s = 0; s < p.n_rk_stages; ++s)
             rk[s + 1] = p.n_rk_stages == 3 ? t3[o][s] : p.n_rk_stages == 4 ? t4[o][s] : t5[o][s];
     }
-    // explicit mixed precision (FP32 staging): smaller tiles and CTAs, six
-    // per SM (0.366 against 0.393 ms per RK3 step at 256 x 256 on the
-    // 500k-triangle double Mach reflection)
-    if (p.precision == CCFD_MIXED && !p.implicit) ctx->tile_cells = 192;
     const char* tc = getenv("CCFD_TILE_CELLS");
     if (tc) ctx->tile_cells = std::max(32, std::min(2048, atoi(tc)));
     const char* th = getenv("CCFD_STAGE_THREADS");
@@ -249,16 +247,25 @@ static void par_for(long n, Fn fn) {
     for (std::thread& th : pool) th.join();
 }
 
+// Cells per tile when the context sets none.  A large tile repeats fewer
+// border faces, a small one leaves fewer SMs idle: microseconds per RK stage
+// at 48 / 64 / 128 / 256 cells (HLLC, 128 threads): 8,000 cells 13.7 / 15.5 /
+// 18.9 / 26.8, 32,761 cells 14.9 / 15.8 / 19.1 / 27.2, 62,834 cells 23.4 /
+// 20.3 / 20.8 / 27.1, 130,321 cells 35.1 / 33.2 / 31.9 / 32.7; at 128 / 256:
+// 500,000 cells 83.1 / 81.3, 1,048,576 cells 185.6 / 175.1.
+static int default_tile_cells(long n) { return n < 48000 ? 48 : n < 96000 ? 64 : n < 320000 ? 128 : 256; }
+
 // Host staging of an upload, kept per thread from one upload to the next:
 // filling a few hundred MB of freshly allocated host memory per upload cost
 // more in page faults than the work itself.
 struct UploadScratch {
-    std::vector<int> cperm, cinv, fint, fdev, cnt, hs_off, hs_nb, hs_dev_of_ref;
-    std::vector<int> g_cell, g_hs, g_bc, gl_off;
-    std::vector<double4> hs_gw, cell_geo, cell_xq, face_nl, face_bb, g_gn, g_ml, g_bb;
-    std::vector<double> venk, e2;
-    std::vector<int4> counts;
-    std::vector<short> hs_nbl, hs_loc;
+    std::vector<int> cperm, cinv, hs_off, hs_nb, ghost_of, g_bc;
+    std::vector<double4> hs_gw, cell_geo, cell_xq, f_nl, f_gp, f_bb, g_gn;
+    std::vector<double2> g_mid;
+    std::vector<double> venk, area_q;
+    std::vector<int4> nb4, slot4, rng, g_list;
+    std::vector<int2> g_rng;
+    std::vector<ushort4> u_code;
     TileSet ts;
 };
 static thread_local UploadScratch tl_upload;
@@ -293,40 +300,19 @@ extern "C" int ccfd_upload_case(ccfd_ctx* ctx, const ccfd_mesh* m, const ccfd_bc
     ctx->cell_of_dev = cperm;
     ctx->dev_of_cell = cinv;
 
-    // interior faces in the order of their owner's device index
-    // (stable counting sort by the owner's device index)
-    std::vector<int>& fint = S.fint;
-    {
-        std::vector<int>& cnt = S.cnt;
-        cnt.assign(N + 1, 0);
-        long nfi = 0;
-        for (long f = 0; f < F; ++f)
-            if (m->face_cells[2 * f + 1] >= 0) {
-                ++cnt[cinv[m->face_cells[2 * f]] + 1];
-                ++nfi;
-            }
-        for (long d = 0; d < N; ++d) cnt[d + 1] += cnt[d];
-        fint.resize(nfi);
-        for (long f = 0; f < F; ++f)
-            if (m->face_cells[2 * f + 1] >= 0) fint[cnt[cinv[m->face_cells[2 * f]]]++] = (int)f;
-    }
-    std::vector<int>& fdev = S.fdev;
-    fdev.assign(F, -1);
-    for (size_t i = 0; i < fint.size(); ++i) fdev[fint[i]] = (int)i;
-    const long FI = (long)fint.size();
-    ctx->F = FI;
-
     // per-cell CSR in device order
     std::vector<int>& hs_off = S.hs_off;
     std::vector<int>& hs_nb = S.hs_nb;
     std::vector<double4>& hs_gw = S.hs_gw;
     std::vector<double4>& cell_geo = S.cell_geo;
     std::vector<double4>& cell_xq = S.cell_xq;
-    std::vector<int>& hs_dev_of_ref = S.hs_dev_of_ref;
+    std::vector<int4>& nb4 = S.nb4;
+    std::vector<double>& area_q = S.area_q;
     hs_off.resize(N + 1);
     cell_geo.resize(N);
     cell_xq.resize(N);
-    hs_dev_of_ref.resize(m->n_half_sides);
+    nb4.resize(N);
+    area_q.resize(N);
     hs_off[0] = 0;
     for (long d = 0; d < N; ++d) {
         long c = cperm[d];
@@ -341,14 +327,17 @@ extern "C" int ccfd_upload_case(ccfd_ctx* ctx, const ccfd_mesh* m, const ccfd_bc
         for (long d = d0; d < d1; ++d) {
             long c = cperm[d];
             long k = hs_off[d];
+            nb4[d] = make_int4(kNoSide, kNoSide, kNoSide, kNoSide);
+            int* nbk = &nb4[d].x;
             for (long h = m->hs_offset[c]; h < m->hs_offset[c + 1]; ++h, ++k) {
                 long nb = m->hs_nb[h];
-                hs_dev_of_ref[h] = (int)k;
                 hs_nb[k] = nb >= 0 ? cinv[nb] : (int)nb;
+                *nbk++ = hs_nb[k];
                 hs_gw[k] = make_double4(m->hs_gp[2 * h], m->hs_gp[2 * h + 1], m->hs_w[2 * h], m->hs_w[2 * h + 1]);
             }
             cell_geo[d] = make_double4(m->cell_geo[4 * c], m->cell_geo[4 * c + 1], m->cell_geo[4 * c + 2],
                                        m->cell_geo[4 * c + 3]);
+            area_q[d] = m->cell_geo[4 * c + 1];
             const double* b = &m->cell_bary[2 * c];
             const double* q5 = m->cell_gp5 ? &m->cell_gp5[2 * c] : b;
             cell_xq[d] = make_double4(b[0], b[1], q5[0], q5[1]);
@@ -357,55 +346,83 @@ extern "C" int ccfd_upload_case(ccfd_ctx* ctx, const ccfd_mesh* m, const ccfd_bc
             venk[d] = vk ? (p.venk_k * sqrt(a)) * (p.venk_k * sqrt(a)) * (p.venk_k * sqrt(a)) : 0.0;
         }
     });
-    // face geometry; the barycentre vectors only for the viscous fluxes
-    const bool ns = p.eqn == CCFD_NAVIER_STOKES;
-    std::vector<double4>& face_nl = S.face_nl;
-    std::vector<double4>& face_bb = S.face_bb;
-    face_nl.resize(FI + 1);
-    face_bb.resize(ns ? FI + 1 : 1);
-    face_nl[FI] = face_bb[face_bb.size() - 1] = make_double4(0, 0, 0, 0);
-    par_for(FI, [&](long i0, long i1) {
-        for (long i = i0; i < i1; ++i) {
-            long f = fint[i];
-            face_nl[i] = make_double4(m->face_n[2 * f], m->face_n[2 * f + 1], m->face_len[f], 0.0);
-            if (ns) face_bb[i] = make_double4(m->face_bb[3 * f], m->face_bb[3 * f + 1], m->face_bb[3 * f + 2], 0.0);
-        }
-    });
     // ghosts (BCside order)
-    std::vector<int>& g_cell = S.g_cell;
-    std::vector<int>& g_hs = S.g_hs;
+    const bool ns = p.eqn == CCFD_NAVIER_STOKES;
     std::vector<int>& g_bc = S.g_bc;
+    std::vector<int>& ghost_of = S.ghost_of;  // boundary face -> ghost
     std::vector<double4>& g_gn = S.g_gn;
-    std::vector<double4>& g_ml = S.g_ml;
-    std::vector<double4>& g_bb = S.g_bb;
-    g_cell.assign(B + 1, 0);
-    g_hs.assign(B + 1, 0);
+    std::vector<double2>& g_mid = S.g_mid;
     g_bc.assign(B + 1, 0);
     g_gn.assign(B + 1, make_double4(0, 0, 0, 0));
-    g_ml.assign(B + 1, make_double4(0, 0, 0, 0));
-    g_bb.assign(B + 1, make_double4(0, 0, 0, 0));
+    g_mid.assign(B + 1, make_double2(0, 0));
+    ghost_of.assign(F, 0);
     for (long g = 0; g < B; ++g) {
         long f = m->bc_face[g];
-        g_cell[g] = cinv[m->face_cells[2 * f]];
-        g_hs[g] = hs_dev_of_ref[m->face_hs[2 * f]];
+        ghost_of[f] = (int)g;
         g_bc[g] = m->bc_index[g];
         g_gn[g] = make_double4(m->bc_ghost_bary[2 * g], m->bc_ghost_bary[2 * g + 1], m->face_n[2 * f],
                                m->face_n[2 * f + 1]);
-        g_ml[g] = make_double4(m->bc_x[2 * g], m->bc_x[2 * g + 1], m->face_len[f], 0.0);
-        g_bb[g] = make_double4(m->face_bb[3 * f], m->face_bb[3 * f + 1], m->face_bb[3 * f + 2], 0.0);
+        g_mid[g] = make_double2(m->bc_x[2 * g], m->bc_x[2 * g + 1]);
     }
-    // tiles of the fused stage kernel
+    // tiles of the flux kernel and the face records in tile order
     TileSet& ts = S.ts;
-    ccfd_build_tiles(m, cperm, cinv, fdev, ctx->tile_cells, ts);
-    if (ts.max_e >= 32768 || ts.max_hs >= 32768) return CCFD_ERR_ARG;
-    std::vector<int4>& counts = S.counts;
-    std::vector<int>& gl_off = S.gl_off;
-    counts.resize(ts.n_tiles);
-    gl_off.assign(ts.n_tiles + 1, 0);
-    for (int t = 0; t < ts.n_tiles; ++t) {
-        counts[t] = make_int4(ts.counts[4 * t], ts.counts[4 * t + 1], ts.counts[4 * t + 2], ts.counts[4 * t + 3]);
-        gl_off[t + 1] = gl_off[t] + ts.counts[4 * t + 1] + 1;
+    ccfd_build_tiles(m, cperm, cinv, ctx->tile_cells > 0 ? ctx->tile_cells : default_tile_cells(N), ts);
+    const bool second = p.spatial_order == 2;
+    std::vector<int4>& rng = S.rng;
+    std::vector<int4>& slot4 = S.slot4;
+    std::vector<double4>& f_nl = S.f_nl;
+    std::vector<double4>& f_gp = S.f_gp;
+    std::vector<double4>& f_bb = S.f_bb;  // only for the viscous fluxes
+    std::vector<ushort4>& u_code = S.u_code;
+    rng.resize(ts.n_tiles);
+    for (int t = 0; t < ts.n_tiles; ++t)
+        rng[t] = make_int4(ts.own_off[t], ts.own_off[t + 1] - ts.own_off[t], ts.border_off[t],
+                           ts.border_off[t + 1] - ts.border_off[t]);
+    f_nl.resize(F);
+    f_gp.resize(ns && second ? F : 0);
+    f_bb.resize(ns ? F : 0);
+    par_for(F, [&](long i0, long i1) {
+        for (long i = i0; i < i1; ++i) {
+            const long f = ts.face_of[i], nb = m->face_cells[2 * f + 1];
+            const int lr[2] = {cinv[m->face_cells[2 * f]], nb >= 0 ? cinv[nb] : -1 - ghost_of[f]};
+            double w;
+            memcpy(&w, lr, sizeof(w));
+            f_nl[i] = make_double4(m->face_n[2 * f], m->face_n[2 * f + 1], m->face_len[f], w);
+            if (ns && second) {
+                const double* gl = &m->hs_gp[2 * m->face_hs[2 * f]];
+                const double* gr = nb >= 0 ? &m->hs_gp[2 * m->face_hs[2 * f + 1]] : gl;
+                f_gp[i] = make_double4(gl[0], gl[1], gr[0], gr[1]);
+            }
+            if (ns) f_bb[i] = make_double4(m->face_bb[3 * f], m->face_bb[3 * f + 1], m->face_bb[3 * f + 2], 0.0);
+        }
+    });
+    // ghosts by tile (of their cell), counting sort
+    std::vector<int2>& g_rng = S.g_rng;
+    std::vector<int4>& g_list = S.g_list;
+    g_rng.assign(ts.n_tiles, make_int2(0, 0));
+    g_list.resize(B);
+    for (long g = 0; g < B; ++g) ++g_rng[cinv[m->face_cells[2 * m->bc_face[g]]] / ts.tile_cells].y;
+    for (int t = 1; t < ts.n_tiles; ++t) g_rng[t].x = g_rng[t - 1].x + g_rng[t - 1].y;
+    for (int2& r : g_rng) r.y = 0;
+    for (long g = 0; g < B; ++g) {
+        const long f = m->bc_face[g];
+        const int d = cinv[m->face_cells[2 * f]];
+        int2& r = g_rng[d / ts.tile_cells];
+        g_list[r.x + r.y++] = make_int4((int)g, d, 2 * ts.id_of[f], 0);
     }
+    // slots of the reconstructed side states (owner's side first)
+    slot4.resize(ns || !second ? 0 : N);
+    u_code.resize(N);
+    par_for(N, [&](long d0, long d1) {
+        memcpy(u_code.data() + d0, &ts.u_code[4 * d0], sizeof(ushort4) * (d1 - d0));
+        for (long d = d0; d < d1 && !slot4.empty(); ++d) {
+            const long c = cperm[d];
+            slot4[d] = make_int4(-1, -1, -1, -1);
+            int* s4 = &slot4[d].x;
+            for (long h = m->hs_offset[c]; h < m->hs_offset[c + 1]; ++h)
+                *s4++ = 2 * ts.id_of[m->hs_face[h]] + (m->hs_sign[h] > 0 ? 0 : 1);
+        }
+    });
     int st;
     DevMesh& dm = ctx->mesh;
     memset(&dm, 0, sizeof(dm));
@@ -413,23 +430,16 @@ extern "C" int ccfd_upload_case(ccfd_ctx* ctx, const ccfd_mesh* m, const ccfd_bc
     memset(&td, 0, sizeof(td));
     GhostDev& gd = ctx->ghosts;
     memset(&gd, 0, sizeof(gd));
-    std::vector<short>& hs_nbl = S.hs_nbl;
-    std::vector<short>& hs_loc = S.hs_loc;
-    hs_nbl.assign(ts.hs_nbl.begin(), ts.hs_nbl.end());
-    hs_loc.assign(ts.hs_loc.begin(), ts.hs_loc.end());
     if ((st = dupload_c(ctx, &dm.hs_off, hs_off)) || (st = dupload_c(ctx, &dm.hs_nb, hs_nb)) ||
-        (st = dupload_c(ctx, &dm.hs_gw, hs_gw)) || (st = dupload_c(ctx, &dm.cell_geo, cell_geo)) ||
-        (st = dupload_c(ctx, &dm.venk_eps2, venk)) || (st = dupload_c(ctx, &dm.face_nl, face_nl)) ||
-        (st = dupload_c(ctx, &dm.face_bb, face_bb)) || (st = dupload_c(ctx, &gd.cell, g_cell)) ||
-        (st = dupload_c(ctx, &gd.hs, g_hs)) || (st = dupload_c(ctx, &gd.bc, g_bc)) ||
-        (st = dupload_c(ctx, &gd.gn, g_gn)) || (st = dupload_c(ctx, &gd.ml, g_ml)) ||
-        (st = dupload_c(ctx, &gd.bb, g_bb)) || (st = dupload_c(ctx, &td.e_off, ts.e_off)) ||
-        (st = dupload_c(ctx, &td.counts, counts)) || (st = dupload_c(ctx, &td.e_ref, ts.e_ref)) ||
-        (st = dupload_c(ctx, &td.hs_off, ts.hs_off)) || (st = dupload_c(ctx, &td.hs_nbl, hs_nbl)) ||
-        (st = dupload_c(ctx, &td.gl_off, gl_off)) || (st = dupload_c(ctx, &td.hs_loc, hs_loc)) ||
-        (st = dupload_c(ctx, &td.f_off, ts.f_off)) || (st = dupload_c(ctx, &td.f_id, ts.f_id)) ||
-        (st = dupload_c(ctx, &td.f_lr, ts.f_lr)) || (st = dupload_c(ctx, &td.f_hs, ts.f_hs)) ||
-        (st = dupload_c(ctx, &td.u_code, ts.u_code)) || (st = dupload_c(ctx, &ctx->cell_xq, cell_xq))) {
+        (st = dupload_c(ctx, &dm.nb4, nb4)) || (st = dupload_c(ctx, &dm.slot4, slot4)) || (st = dupload_c(ctx, &dm.hs_gw, hs_gw)) ||
+        (st = dupload_c(ctx, &dm.cell_geo, cell_geo)) || (st = dupload_c(ctx, &dm.area_q, area_q)) ||
+        (st = dupload_c(ctx, &dm.venk_eps2, venk)) || (st = dupload_c(ctx, &gd.bc, g_bc)) ||
+        (st = dupload_c(ctx, &gd.gn, g_gn)) || (st = dupload_c(ctx, &gd.mid, g_mid)) ||
+        (st = dalloc(ctx, &gd.state, (size_t)B + 1)) || (st = dalloc(ctx, &gd.face, (size_t)B + 1)) || (st = dupload_c(ctx, &td.rng, rng)) ||
+        (st = dupload_c(ctx, &td.border, ts.border)) ||
+        (st = dupload_c(ctx, &td.g_rng, g_rng)) || (st = dupload_c(ctx, &td.ghost, g_list)) || (st = dupload_c(ctx, &td.f_nl, f_nl)) ||
+        (st = dupload_c(ctx, &td.f_gp, f_gp)) || (st = dupload_c(ctx, &td.f_bb, f_bb)) ||
+        (st = dupload_c(ctx, &td.u_code, u_code)) || (st = dupload_c(ctx, &ctx->cell_xq, cell_xq))) {
         free_device(ctx);
         return st;
     }
@@ -441,19 +451,18 @@ extern "C" int ccfd_upload_case(ccfd_ctx* ctx, const ccfd_mesh* m, const ccfd_bc
         }
     }
     dm.N = (int)N;
-    dm.F = (int)FI;
+    dm.F = (int)(F - B);
     dm.B = (int)B;
     dm.H = hs_off[N];
     td.n_tiles = ts.n_tiles;
-    td.max_e = ts.max_e;
-    td.max_g = ts.max_g;
-    td.max_hs = ts.max_hs;
+    td.cells = ts.tile_cells;
     td.max_f = ts.max_f;
-    td.smem_bytes = stage_smem_bytes(td, 0);  // FP64 staging: the larger of the two layouts
     td.threads = ctx->stage_threads;
     int smem_max = 0;
     CK(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
-    if (td.smem_bytes > smem_max) {
+    // FP64 fluxes: the larger of the two layouts; 16 KB are left for the
+    // kernel's static shared memory
+    if (stage_smem_bytes(td.max_f, 0) > smem_max - 16384) {
         free_device(ctx);
         return CCFD_ERR_ARG;
     }
@@ -513,6 +522,7 @@ extern "C" int ccfd_upload_case(ccfd_ctx* ctx, const ccfd_mesh* m, const ccfd_bc
     }
 
     // state and scratch
+    const bool fp32_only = p.precision == CCFD_MIXED && !p.implicit;
     ctx->nb_cells = (int)((N + 255) / 256);
     ctx->nb_part = std::max(ctx->nb_cells, ts.n_tiles);
     if ((st = dupload_c(ctx, &ctx->d_cell_of_dev, ctx->cell_of_dev)) ||
@@ -520,6 +530,10 @@ extern "C" int ccfd_upload_case(ccfd_ctx* ctx, const ccfd_mesh* m, const ccfd_bc
         (st = dalloc(ctx, &ctx->prim_buf[0], N)) || (st = dalloc(ctx, &ctx->prim_buf[1], N)) ||
         (st = dalloc(ctx, &ctx->cons0, N)) || (st = dalloc(ctx, &ctx->u_t, N)) ||
         (st = dalloc(ctx, &ctx->grad, 2 * N)) || (st = dalloc(ctx, &ctx->ticket, 1)) ||
+        // reconstructed face states (Euler; half the bytes when only the FP32
+        // scheme uses them), FP32 gradients of the explicit viscous scheme
+        (second && !ns && (st = dalloc(ctx, &ctx->fstate, (fp32_only ? 1 : 2) * (size_t)F))) ||
+        (second && ns && fp32_only && (st = dalloc(ctx, &ctx->grad_f, 2 * (size_t)N))) ||
         (st = dalloc(ctx, &ctx->ghost_pface, B + 1)) ||
         (st = dalloc(ctx, &ctx->flags, 1)) || (st = dalloc(ctx, &ctx->ctrl, 1)) ||
         (st = dalloc(ctx, &ctx->dt_partial, ctx->nb_part)) || (st = dalloc(ctx, &ctx->dt_bad, ctx->nb_part)) ||
@@ -596,7 +610,7 @@ void ccfd_fill_stage(ccfd_ctx* ctx, StageLaunch& L) {
     L.mesh = ctx->mesh;
     L.tiles = ctx->tiles;
     L.ghosts = ctx->ghosts;
-    L.phys = ctx->phys;
+    L.gas = ctx->phys;
     L.phys_g = ctx->phys_g;
     L.sp = ctx->sp;
     L.order = ctx->params.spatial_order;
@@ -607,6 +621,10 @@ void ccfd_fill_stage(ccfd_ctx* ctx, StageLaunch& L) {
     // scheme keeps FP64 residuals (its finite-difference Jacobian-vector
     // products divide residual differences by a tiny perturbation)
     L.fp32 = ctx->params.precision == CCFD_MIXED && !ctx->params.implicit;
+    L.prim_buf[0] = ctx->prim_buf[0];
+    L.prim_buf[1] = ctx->prim_buf[1];
+    L.grad = ctx->grad_f ? (void*)ctx->grad_f : (void*)ctx->grad;
+    L.fstate = ctx->fstate;
     L.ghost_pface = ctx->ghost_pface;
     L.flags = ctx->flags;
     L.ticket = ctx->ticket;
@@ -710,8 +728,16 @@ extern "C" int ccfd_get_time(ccfd_ctx* ctx, double* t) {
     return CCFD_OK;
 }
 
-// Residual of the current state into ctx->u_t (device); no host copies.
-int ccfd_residual_device(ccfd_ctx* ctx, double time) {
+// where k_grad writes the gradients for the caller (ctx->grad): the FP64
+// viscous scheme keeps them there anyway
+static double4* grad_out_of(ccfd_ctx* ctx) {
+    const bool kept = ctx->params.eqn == CCFD_NAVIER_STOKES && !ctx->grad_f;
+    return ctx->params.spatial_order == 2 && !kept ? ctx->grad : nullptr;
+}
+
+// Residual of the current state into ctx->u_t (and, with want_grad, its
+// limited gradients into ctx->grad) on the device; no host copies.
+int ccfd_residual_device(ccfd_ctx* ctx, double time, bool want_grad) {
     StageLaunch L;
     ccfd_fill_stage(ctx, L);
     L.ctrl = nullptr;
@@ -719,7 +745,7 @@ int ccfd_residual_device(ccfd_ctx* ctx, double time) {
     L.mode = 0;
     L.prim_in = cur_prim(ctx);
     L.u_t = ctx->u_t;
-    L.grad_out = ctx->params.spatial_order == 2 ? ctx->grad : nullptr;
+    L.grad_out = want_grad ? grad_out_of(ctx) : nullptr;
     L.res_partial = ctx->res_partial;
     launch_stage(L, ctx->stream);
     CK(cudaGetLastError());
@@ -744,7 +770,7 @@ extern "C" int ccfd_residual(ccfd_ctx* ctx, double time, double* u_t_out, double
     if (!ctx || !ctx->uploaded) return CCFD_ERR_ARG;
     if (ctx->batch) return CCFD_ERR_BUSY;
     CK(cudaSetDevice(ctx->device));
-    int st = ccfd_residual_device(ctx, time);
+    int st = ccfd_residual_device(ctx, time, grad_out != nullptr);
     if (st) return st;
     const long N = ctx->N;
     if (u_t_out) {
@@ -762,16 +788,16 @@ extern "C" int ccfd_residual(ccfd_ctx* ctx, double time, double* u_t_out, double
         CK(cudaStreamSynchronize(ctx->stream));
         for (long d = 0; d < N; ++d) {
             double* s = &grad_out[8 * ctx->cell_of_dev[d]];
-            s[0] = h[2 * d].x; s[1] = h[2 * d].y; s[2] = h[2 * d].z; s[3] = h[2 * d].w;
-            s[4] = h[2 * d + 1].x; s[5] = h[2 * d + 1].y; s[6] = h[2 * d + 1].z; s[7] = h[2 * d + 1].w;
+            // stored variable by variable (ld_grad in stage_impl.cuh)
+            s[0] = h[2 * d].x; s[1] = h[2 * d].z; s[2] = h[2 * d + 1].x; s[3] = h[2 * d + 1].z;
+            s[4] = h[2 * d].y; s[5] = h[2 * d].w; s[6] = h[2 * d + 1].y; s[7] = h[2 * d + 1].w;
         }
     }
     return check_flags(ctx);
 }
 
 // calcErrors (src/analyze.c:445-514) at the current time: the limited
-// gradients of the current state (spatialReconstruction, as one residual
-// evaluation that writes only the gradients), then the per-cell quadrature
+// gradients of the current state (spatialReconstruction), then the per-cell quadrature
 // errors against exact function `exact_func` and the CTA partials summed
 // here in CTA order.
 extern "C" int ccfd_errors(ccfd_ctx* ctx, int exact_func, double out[12]) {
@@ -789,11 +815,8 @@ extern "C" int ccfd_errors(ccfd_ctx* ctx, int exact_func, double out[12]) {
         L.tfix = t;
         L.mode = 0;
         L.prim_in = cur_prim(ctx);
-        L.u_t = nullptr;
-        L.grad_out = ctx->grad;
-        L.res_partial = nullptr;
-        L.ghost_pface = nullptr;
-        launch_stage(L, ctx->stream);
+        L.grad_out = grad_out_of(ctx);
+        launch_gradients(L, ctx->stream);
         CK(cudaGetLastError());
     }
     const int nb = error_blocks((int)ctx->N);
@@ -967,10 +990,10 @@ extern "C" int ccfd_autotune(ccfd_ctx* ctx, const ccfd_mesh* m, const ccfd_bc* b
             // the CTA size changes the launch only: time each on the same tiles
             for (int k = 0; k < 3; ++k) {
                 ctx->tiles.threads = thr_list[k];
-                if ((st = ccfd_residual_device(ctx, 0.0))) return st;  // warm-up
+                if ((st = ccfd_residual_device(ctx, 0.0, false))) return st;  // warm-up
                 CK(cudaEventRecord(ev.a, ctx->stream));
                 for (int r = 0; r < kReps; ++r)
-                    if ((st = ccfd_residual_device(ctx, 0.0))) return st;
+                    if ((st = ccfd_residual_device(ctx, 0.0, false))) return st;
                 CK(cudaEventRecord(ev.b, ctx->stream));
                 CK(cudaEventSynchronize(ev.b));
                 float ms = 0.0f;

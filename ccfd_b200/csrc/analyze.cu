@@ -34,8 +34,9 @@ __global__ void __launch_bounds__(kErrThreads)
         double gx[4] = {0, 0, 0, 0}, gy[4] = {0, 0, 0, 0};
         if (grad) {
             const double4 a = grad[2 * d], b = grad[2 * d + 1];
-            gx[0] = a.x; gx[1] = a.y; gx[2] = a.z; gx[3] = a.w;
-            gy[0] = b.x; gy[1] = b.y; gy[2] = b.z; gy[3] = b.w;
+            // stored variable by variable (ld_grad in stage_impl.cuh)
+            gx[0] = a.x; gy[0] = a.y; gx[1] = a.z; gy[1] = a.w;
+            gx[2] = b.x; gy[2] = b.y; gx[3] = b.z; gy[3] = b.w;
         }
         for (int k = 0; k < ns + (quad ? 1 : 0); ++k) {
             double x[2], wk;

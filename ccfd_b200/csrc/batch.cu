@@ -29,8 +29,7 @@ struct VariantGroup {
     std::vector<int> members;  // indices into ccfd_batch::inst
     int n_tiles = 0, smem_bytes = 0;
     StageLaunch* d_recs = nullptr;
-    int2* d_tmap = nullptr;
-    int* d_ctr = nullptr;  // tile claim counters of the group's launches
+    int4* d_tmap = nullptr;
 };
 
 __global__ void k_gather_ctrl(const Ctrl* const* __restrict__ src, Ctrl* __restrict__ dst, int n) {
@@ -82,7 +81,6 @@ static void drop_group_memory(ccfd_batch* b) {
     for (auto& g : b->groups) {
         if (g.d_recs) cudaFreeAsync(g.d_recs, b->stream);
         if (g.d_tmap) cudaFreeAsync(g.d_tmap, b->stream);
-        if (g.d_ctr) cudaFreeAsync(g.d_ctr, b->stream);
     }
     b->groups.clear();
     for (auto& g : b->graph)
@@ -92,30 +90,17 @@ static void drop_group_memory(ccfd_batch* b) {
         }
 }
 
-// launch records of member ctx: [parity][stage] for the RK stages
-static void member_records(ccfd_ctx* ctx, StageLaunch* out) {
-    const StepParams& sp = ctx->sp;
-    for (int par = 0; par < 2; ++par)
-        for (int s = 0; s < kBatchStages; ++s) {
-            StageLaunch& L = out[par * kBatchStages + s];
-            ccfd_fill_stage(ctx, L);
-            L.ctrl = ctx->ctrl;
-            if (s >= sp.nrk) {
-                L.mode = -1;
-                continue;
-            }
-            int pin = par ^ (s & 1);
-            L.mode = 1;
-            L.a_time = sp.rk[s];
-            L.rk = sp.rk[s + 1];
-            L.prim_in = ctx->prim_buf[pin];
-            L.prim_out = ctx->prim_buf[pin ^ 1];
-            L.cons0 = ctx->cons0;
-            L.last_stage = s == sp.nrk - 1;
-            L.res_partial = L.last_stage ? ctx->res_partial : nullptr;
-            L.dt_partial = L.last_stage ? ctx->dt_partial : nullptr;
-            L.dt_bad = ctx->dt_bad;
-        }
+// launch record of member ctx for the RK stages: the kernel takes the state
+// buffers, the coefficients and the last stage's outputs from the parity in
+// the control block and the stage number
+static void member_record(ccfd_ctx* ctx, StageLaunch& L) {
+    ccfd_fill_stage(ctx, L);
+    L.ctrl = ctx->ctrl;
+    L.mode = 1;
+    L.cons0 = ctx->cons0;
+    L.res_partial = ctx->res_partial;
+    L.dt_partial = ctx->dt_partial;
+    L.dt_bad = ctx->dt_bad;
 }
 
 // group the explicit members by kernel variant, upload their launch records
@@ -145,28 +130,22 @@ static int rebuild(ccfd_batch* b) {
         b->max_nrk = std::max(b->max_nrk, c->sp.nrk);
     }
     for (auto& g : b->groups) {
-        std::vector<StageLaunch> recs(g.members.size() * 2 * kBatchStages);
-        std::vector<int2> tmap;
-        TileDev big;
-        memset(&big, 0, sizeof(big));
+        std::vector<StageLaunch> recs(g.members.size());
+        std::vector<int4> tmap;
+        int max_f = 0;
         for (size_t k = 0; k < g.members.size(); ++k) {
             ccfd_ctx* c = b->inst[g.members[k]];
-            member_records(c, &recs[k * 2 * kBatchStages]);
-            for (int t = 0; t < c->tiles.n_tiles; ++t) tmap.push_back(make_int2((int)k, t));
-            big.max_e = std::max(big.max_e, c->tiles.max_e);
-            big.max_g = std::max(big.max_g, c->tiles.max_g);
-            big.max_hs = std::max(big.max_hs, c->tiles.max_hs);
-            big.max_f = std::max(big.max_f, c->tiles.max_f);
+            member_record(c, recs[k]);
+            for (int t = 0; t < c->tiles.n_tiles; ++t) tmap.push_back(tile_entry((int)k, t, c->ctrl));
+            max_f = std::max(max_f, c->tiles.max_f);
         }
         g.n_tiles = (int)tmap.size();
-        g.smem_bytes = stage_smem_bytes(big, g.fp32);
+        g.smem_bytes = stage_smem_bytes(max_f, g.fp32);
         CKB(ccfd_malloc_async((void**)&g.d_recs, sizeof(StageLaunch) * recs.size(), b->stream));
-        CKB(ccfd_malloc_async((void**)&g.d_tmap, sizeof(int2) * tmap.size(), b->stream));
-        CKB(ccfd_malloc_async((void**)&g.d_ctr, sizeof(int) * 2, b->stream));
-        CKB(cudaMemsetAsync(g.d_ctr, 0, sizeof(int) * 2, b->stream));
+        CKB(ccfd_malloc_async((void**)&g.d_tmap, sizeof(int4) * tmap.size(), b->stream));
         CKB(cudaMemcpyAsync(g.d_recs, recs.data(), sizeof(StageLaunch) * recs.size(), cudaMemcpyHostToDevice,
                             b->stream));
-        CKB(cudaMemcpyAsync(g.d_tmap, tmap.data(), sizeof(int2) * tmap.size(), cudaMemcpyHostToDevice,
+        CKB(cudaMemcpyAsync(g.d_tmap, tmap.data(), sizeof(int4) * tmap.size(), cudaMemcpyHostToDevice,
                             b->stream));
     }
     while (b->gstream.size() < b->groups.size()) {
@@ -209,7 +188,6 @@ static void launch_steps(ccfd_batch* b, int steps) {
                 BatchLaunch B;
                 B.recs = g.d_recs;
                 B.tmap = g.d_tmap;
-                B.ctr = g.d_ctr;
                 B.n_tiles = g.n_tiles;
                 B.smem_bytes = g.smem_bytes;
                 B.rk_mode = 1;

@@ -18,7 +18,7 @@ struct ccfd_ctx {
     ccfd::DevMesh mesh;
     ccfd::TileDev tiles;
     ccfd::GhostDev ghosts;
-    int tile_cells = 256;
+    int tile_cells = 0;     // cells per tile, 0: by the mesh size
     int stage_threads = 0;  // CTA size of the stage kernel, 0: the precision's default
     ccfd_exact exact;
     double rk[6];
@@ -36,7 +36,9 @@ struct ccfd_ctx {
     int cur = 0;
     double4* cons0 = nullptr;
     double4* u_t = nullptr;
-    double4* grad = nullptr;
+    double4* grad = nullptr;     // [2N] limited gradients, (x, y) variable by variable
+    float4* grad_f = nullptr;    // [2N] FP32 gradients of the explicit mixed-precision viscous scheme
+    double4* fstate = nullptr;   // [2F] reconstructed face states (Euler, second order)
     const double4* cell_xq = nullptr;  // [N] (bary, fifth quad point): source term and error norms
     const int* d_cell_of_dev = nullptr;  // [N] on the device: state transfers permute there
     const int* d_dev_of_cell = nullptr;
@@ -89,7 +91,7 @@ cudaError_t ccfd_malloc_async(void** p, size_t bytes, cudaStream_t st);
 // iteration in ctx->h_ctrl, which the caller has refreshed) to the host
 int ccfd_history_drain(ccfd_ctx* ctx);
 // device-side residual of the current state into ctx->u_t (abi.cu)
-int ccfd_residual_device(ccfd_ctx* ctx, double time);
+int ccfd_residual_device(ccfd_ctx* ctx, double time, bool want_grad);
 // residual of an arbitrary primitive state into ut (abi.cu)
 int ccfd_residual_of(ccfd_ctx* ctx, const double4* prim, double time, double4* ut);
 // implicit solver set-up / release (implicit.cu); the device buffers are

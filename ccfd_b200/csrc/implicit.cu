@@ -1036,8 +1036,8 @@ struct ImpGroup {
     int jac32 = 0;       // Jacobian columns (and their base) with FP32 fluxes (mixed-precision members)
     int n_tiles = 0, smem = 0, smem_jac = 0;
     StageLaunch *rec_mv = nullptr, *rec_nt = nullptr, *rec_jac = nullptr, *rec_jb = nullptr;
-    int2* tmap = nullptr;
-    int* ctr = nullptr;  // tile claim counters of the group's launches
+    // tile maps of the records: the same tiles with each kind's skip word
+    int4 *tmap_mv = nullptr, *tmap_nt = nullptr, *tmap_jac = nullptr;
 };
 
 struct ImpSet {
@@ -1062,8 +1062,9 @@ static void set_free(ImpSet* M) {
         cudaFreeAsync(g.rec_nt, M->stream);
         cudaFreeAsync(g.rec_jac, M->stream);
         cudaFreeAsync(g.rec_jb, M->stream);
-        cudaFreeAsync(g.tmap, M->stream);
-        cudaFreeAsync(g.ctr, M->stream);
+        cudaFreeAsync(g.tmap_mv, M->stream);
+        cudaFreeAsync(g.tmap_nt, M->stream);
+        cudaFreeAsync(g.tmap_jac, M->stream);
     }
     if (M->dev) cudaFreeAsync(M->dev, M->stream);
     if (M->d_count) cudaFreeAsync(M->d_count, M->stream);
@@ -1153,9 +1154,8 @@ static int set_build(const std::vector<ccfd_ctx*>& members, cudaStream_t stream,
         std::tie(g.flux, g.order, g.ns, g.fp32, g.jac32) = kv.first;
         const std::vector<int>& idx = kv.second;
         std::vector<StageLaunch> mv(idx.size()), nt(idx.size()), jac(idx.size()), jb(idx.size());
-        std::vector<int2> tmap;
-        TileDev big;
-        memset(&big, 0, sizeof(big));
+        std::vector<int4> tm_mv, tm_nt, tm_jac;
+        int max_f = 0;
         for (size_t j = 0; j < idx.size(); ++j) {
             ccfd_ctx* ctx = members[idx[j]];
             ImpState* S = (ImpState*)ctx->implicit_state;
@@ -1185,15 +1185,16 @@ static int set_build(const std::vector<ccfd_ctx*>& members, cudaStream_t stream,
             // their base in mixed precision: R(U, t) with FP32 fluxes
             L.u_t = S->RJB;
             jb[j] = L;
-            for (int t = 0; t < ctx->tiles.n_tiles; ++t) tmap.push_back(make_int2((int)j, t));
-            big.max_e = std::max(big.max_e, ctx->tiles.max_e);
-            big.max_g = std::max(big.max_g, ctx->tiles.max_g);
-            big.max_hs = std::max(big.max_hs, ctx->tiles.max_hs);
-            big.max_f = std::max(big.max_f, ctx->tiles.max_f);
+            for (int t = 0; t < ctx->tiles.n_tiles; ++t) {
+                tm_mv.push_back(tile_entry((int)j, t, mv[j].skip));
+                tm_nt.push_back(tile_entry((int)j, t, nt[j].skip));
+                tm_jac.push_back(tile_entry((int)j, t, jac[j].skip));
+            }
+            max_f = std::max(max_f, ctx->tiles.max_f);
         }
-        g.n_tiles = (int)tmap.size();
-        g.smem = stage_smem_bytes(big, g.fp32);
-        g.smem_jac = stage_smem_bytes(big, g.jac32);
+        g.n_tiles = (int)tm_mv.size();
+        g.smem = stage_smem_bytes(max_f, g.fp32);
+        g.smem_jac = stage_smem_bytes(max_f, g.jac32);
         size_t rb = sizeof(StageLaunch) * idx.size();
         CKM(ccfd_malloc_async((void**)&g.rec_mv, rb, stream));
         CKM(ccfd_malloc_async((void**)&g.rec_nt, rb, stream));
@@ -1202,13 +1203,16 @@ static int set_build(const std::vector<ccfd_ctx*>& members, cudaStream_t stream,
             CKM(ccfd_malloc_async((void**)&g.rec_jb, rb, stream));
             CKM(cudaMemcpyAsync(g.rec_jb, jb.data(), rb, cudaMemcpyHostToDevice, stream));
         }
-        CKM(ccfd_malloc_async((void**)&g.tmap, sizeof(int2) * tmap.size(), stream));
-        CKM(ccfd_malloc_async((void**)&g.ctr, sizeof(int) * 2, stream));
-        CKM(cudaMemsetAsync(g.ctr, 0, sizeof(int) * 2, stream));
+        const size_t tb = sizeof(int4) * tm_mv.size();
+        CKM(ccfd_malloc_async((void**)&g.tmap_mv, tb, stream));
+        CKM(ccfd_malloc_async((void**)&g.tmap_nt, tb, stream));
+        CKM(ccfd_malloc_async((void**)&g.tmap_jac, tb, stream));
+        CKM(cudaMemcpyAsync(g.tmap_mv, tm_mv.data(), tb, cudaMemcpyHostToDevice, stream));
+        CKM(cudaMemcpyAsync(g.tmap_nt, tm_nt.data(), tb, cudaMemcpyHostToDevice, stream));
+        CKM(cudaMemcpyAsync(g.tmap_jac, tm_jac.data(), tb, cudaMemcpyHostToDevice, stream));
         CKM(cudaMemcpyAsync(g.rec_mv, mv.data(), rb, cudaMemcpyHostToDevice, stream));
         CKM(cudaMemcpyAsync(g.rec_nt, nt.data(), rb, cudaMemcpyHostToDevice, stream));
         CKM(cudaMemcpyAsync(g.rec_jac, jac.data(), rb, cudaMemcpyHostToDevice, stream));
-        CKM(cudaMemcpyAsync(g.tmap, tmap.data(), sizeof(int2) * tmap.size(), cudaMemcpyHostToDevice, stream));
         M->groups.push_back(g);
     }
     CKM(cudaStreamSynchronize(stream));
@@ -1226,8 +1230,7 @@ static void residuals(ImpSet* M, RecKind kind) {
         const bool jac = kind == REC_JAC || kind == REC_JB;
         BatchLaunch B;
         B.recs = kind == REC_MV ? g.rec_mv : kind == REC_NT ? g.rec_nt : kind == REC_JAC ? g.rec_jac : g.rec_jb;
-        B.tmap = g.tmap;
-        B.ctr = g.ctr;
+        B.tmap = kind == REC_MV ? g.tmap_mv : kind == REC_NT ? g.tmap_nt : g.tmap_jac;
         B.n_tiles = g.n_tiles;
         B.smem_bytes = jac ? g.smem_jac : g.smem;
         B.rk_mode = 0;

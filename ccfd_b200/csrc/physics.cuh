@@ -31,9 +31,16 @@ struct DevExact {
     double x_min, x_max, y_min, y_max, dx_ref;
 };
 
-// Physics constants, passed by value to every kernel (constant bank).
-struct Phys {
-    double gam, gam1, gam1q, mu, Pr, pi, sqrt3q;
+// Gas constants of the fluxes, the update and the time step (part of every
+// launch record).
+struct Gas {
+    double gam, gam1, gam1q, mu, Pr;
+};
+
+// All physics constants; the boundary and exact-solution code reads them
+// from device memory.
+struct Phys : Gas {
+    double pi, sqrt3q;
     int nbc;
     int order;      // spatial order 1 / 2
     int eqn;        // 0 Euler, 1 Navier-Stokes
@@ -461,7 +468,7 @@ struct FluxIn {
 };
 
 // flux_god, src/fluxCalculation.c:30-53 (FP64 only)
-__device__ inline void flux_god(const Phys& P, const FluxIn<double>& s, double f[4],
+__device__ inline void flux_god(const Gas& P, const FluxIn<double>& s, double f[4],
                                 unsigned* flags) {
     double cL = sqrt(P.gam * s.pL / s.rL);
     double cR = sqrt(P.gam * s.pR / s.rR);
@@ -581,7 +588,10 @@ __device__ __forceinline__ void flux_hlle(T gam, T gam1, T gam1q, const FluxIn<T
     hll_tail(arp, alm, fL, fR, uL, uR, f);
 }
 
-// flux_hllc, src/fluxCalculation.c:315-396
+// flux_hllc, src/fluxCalculation.c:315-396.  Whichever region holds the face,
+// the flux is one side's physical flux plus, in the star region, that side's
+// correction: the side is chosen first and only its state and flux are
+// formed (half the live values, no divergent copies of the formulas).
 template <typename T>
 __device__ __forceinline__ void flux_hllc(T gam, T gam1, T gam1q, const FluxIn<T>& s, T f[4]) {
     T rhoLq = T(1.0) / s.rL, rhoRq = T(1.0) / s.rR;
@@ -589,10 +599,6 @@ __device__ __forceinline__ void flux_hllc(T gam, T gam1, T gam1q, const FluxIn<T
     T rhoSqQsum = T(1.0) / (rhoSqL + rhoSqR);
     T eR = gam1q * s.pR + T(0.5) * s.rR * (s.uR * s.uR + s.vR * s.vR);
     T eL = gam1q * s.pL + T(0.5) * s.rL * (s.uL * s.uL + s.vL * s.vL);
-    T uL[4] = {s.rL, s.rL * s.uL, s.rL * s.vL, eL};
-    T uR[4] = {s.rR, s.rR * s.uR, s.rR * s.vR, eR};
-    T fL[4] = {uL[1], uL[1] * s.uL + s.pL, uL[1] * s.vL, s.uL * (eL + s.pL)};
-    T fR[4] = {uR[1], uR[1] * s.uR + s.pR, uR[1] * s.vR, s.uR * (eR + s.pR)};
     T cL = sqrt(gam * s.pL * rhoLq), cR = sqrt(gam * s.pR * rhoRq);
     T HL = (eL + s.pL) * rhoLq, HR = (eR + s.pR) * rhoRq;
     T uM = (rhoSqR * s.uR + rhoSqL * s.uL) * rhoSqQsum;
@@ -601,28 +607,28 @@ __device__ __forceinline__ void flux_hllc(T gam, T gam1, T gam1q, const FluxIn<T
     T cM = sqrt(gam1 * (HM - T(0.5) * (uM * uM + vM * vM)));
     T arp = fmax(s.uR + cR, uM + cM);
     T alm = fmin(s.uL - cL, uM - cM);
-    if (alm > T(0.0)) {
+    const bool star = !(alm > T(0.0)) && !(arp < T(0.0));
+    bool left = alm > T(0.0);
+    T as = T(0.0);
+    if (star) {
+        as = (s.pR - s.pL + s.rL * s.uL * (alm - s.uL) - s.rR * s.uR * (arp - s.uR)) /
+             (s.rL * (alm - s.uL) - s.rR * (arp - s.uR));
+        left = (alm <= T(0.0)) && (as >= T(0.0));
+    }
+    const T rk = left ? s.rL : s.rR, uk = left ? s.uL : s.uR, vk = left ? s.vL : s.vR, pk = left ? s.pL : s.pR,
+            ek = left ? eL : eR;
+    const T mk = rk * uk;
+    f[0] = mk;
+    f[1] = mk * uk + pk;
+    f[2] = mk * vk;
+    f[3] = uk * (ek + pk);
+    if (star) {
+        const T sk = left ? alm : arp;
+        const T fac = rk * (sk - uk) / (sk - as);
+        const T us[4] = {fac, as * fac, vk * fac, fac * (ek / rk + (as - uk) * (as + pk / (rk * (sk - uk))))};
+        const T uv[4] = {rk, mk, rk * vk, ek};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) f[i] = fL[i];
-    } else if (arp < T(0.0)) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) f[i] = fR[i];
-    } else {
-        T as = (s.pR - s.pL + uL[1] * (alm - s.uL) - uR[1] * (arp - s.uR)) /
-               (s.rL * (alm - s.uL) - s.rR * (arp - s.uR));
-        if ((alm <= T(0.0)) && (as >= T(0.0))) {
-            T fac = s.rL * (alm - s.uL) / (alm - as);
-            T us[4] = {fac, as * fac, s.vL * fac,
-                       fac * (eL / s.rL + (as - s.uL) * (as + s.pL / (s.rL * (alm - s.uL))))};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) f[i] = fL[i] + alm * (us[i] - uL[i]);
-        } else {
-            T fac = s.rR * (arp - s.uR) / (arp - as);
-            T us[4] = {fac, as * fac, s.vR * fac,
-                       fac * (eR / s.rR + (as - s.uR) * (as + s.pR / (s.rR * (arp - s.uR))))};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) f[i] = fR[i] + arp * (us[i] - uR[i]);
-        }
+        for (int i = 0; i < 4; ++i) f[i] = f[i] + sk * (us[i] - uv[i]);
     }
 }
 
@@ -798,7 +804,7 @@ __device__ __forceinline__ void flux_vanleer(T gam, T gam1, T gam1q, const FluxI
 // convectiveFlux dispatch, src/fluxCalculation.c:803-844 (FLUX is a template
 // constant, so each kernel instantiation carries exactly one flux)
 template <int FLUX, typename T>
-__device__ __forceinline__ void convective_flux(const Phys& P, const FluxIn<T>& s, T f[4],
+__device__ __forceinline__ void convective_flux(const Gas& P, const FluxIn<T>& s, T f[4],
                                                 unsigned* flags) {
     const T gam = T(P.gam), gam1 = T(P.gam1), gam1q = T(P.gam1q);
     if constexpr (FLUX == 1) {
@@ -833,7 +839,7 @@ __device__ __forceinline__ void convective_flux(const Phys& P, const FluxIn<T>& 
 // diffusionFlux, src/fluxCalculation.c:855-873 (state: mean primitive state,
 // gx / gy: face gradients of the primitive variables); f[0] = g[0] = 0
 template <typename T>
-__device__ __forceinline__ void diffusion_flux(const Phys& P, const T st[4], const T gx[4],
+__device__ __forceinline__ void diffusion_flux(const Gas& P, const T st[4], const T gx[4],
                                                const T gy[4], T f[4], T g[4]) {
     const T mu = T(P.mu), c43 = T(4.0 / 3.0), c23 = T(2.0 / 3.0);
     const T gam = T(P.gam), gam1 = T(P.gam1), Pr = T(P.Pr);

@@ -10,15 +10,18 @@ namespace ccfd {
 
 // Mesh in device memory, uploaded once: cells in Hilbert order, 32-bit
 // indices, 32-byte records so that every gather of a record is one sector.
+constexpr int kNoSide = 0x7fffffff;  // fourth side of a triangle in DevMesh::nb4
+
 struct DevMesh {
     int N, F, B, H;           // cells, interior faces, ghosts, half-sides
     const int* hs_off;        // [N+1] CSR offsets of the per-cell half-sides
     const int* hs_nb;         // [H] neighbour cell, or -1-g for ghost g
+    const int4* nb4;          // [N] the same per cell in side order, kNoSide padded
+    const int4* slot4;        // [N] per side the slot (2 face + side) of its state (Euler, second order)
     const double4* hs_gw;     // [H] (GP.x, GP.y, w.x, w.y)
     const double4* cell_geo;  // [N] (area, 1/area, sx, sy)
+    const double* area_q;     // [N] 1/area
     const double* venk_eps2;  // [N] Venkatakrishnan epsilon^2
-    const double4* face_nl;   // [F] (n.x, n.y, len, 0) of interior faces
-    const double4* face_bb;   // [F] (baryBaryVec.x, .y, baryBaryDist, 0)
     const double4* cell_src;  // [N] (bary, fifth quad point) when the source term is on, else nullptr
     double4* src_buf;         // [N] the cells' source term of the running evaluation (with cell_src)
 };

@@ -11,7 +11,7 @@ namespace ccfd {
 
 // per-block minima of the convective and viscous time steps; the CFL
 // number is the control block's under switched evolution relaxation
-__global__ void __launch_bounds__(256) k_dt(DevMesh m, Phys P, const Ctrl* ctrl, StepParams sp,
+__global__ void __launch_bounds__(256) k_dt(DevMesh m, Gas P, const Ctrl* ctrl, StepParams sp,
                                             const double4* __restrict__ prim,
                                             double2* __restrict__ partial, int* bad_partial) {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -94,7 +94,7 @@ __global__ void k_step_dt(Ctrl* ctrl, StepParams sp, const double2* __restrict__
     finish_dt(ctrl, sp, a, b, bad);
 }
 
-void imp_step_end_launch(Ctrl* ctrl, const DevMesh& m, const Phys& P, const StepParams& sp,
+void imp_step_end_launch(Ctrl* ctrl, const DevMesh& m, const Gas& P, const StepParams& sp,
                          const double* res_partial, int nres, double2* dt_partial, int* dt_bad, int ndt,
                          const int* wall_ghost, const double* wall_nl, const double* ghost_pface,
                          const double4* prim_new, cudaStream_t st) {
@@ -105,11 +105,18 @@ void imp_step_end_launch(Ctrl* ctrl, const DevMesh& m, const Phys& P, const Step
 
 
 // ------------------------------------------------------------ dispatchers
-int stage_smem_bytes(const TileDev& T, int fp32) {
-    return fp32 ? stage_smem_bytes_t<float>(T) : stage_smem_bytes_t<double>(T);
+int stage_smem_bytes(int max_f, int fp32) {
+    return fp32 ? stage_smem_bytes_t<float>(max_f, StageShape<float>::single)
+                : stage_smem_bytes_t<double>(max_f, StageShape<double>::single);
+}
+
+void launch_gradients(const StageLaunch& L, cudaStream_t st) {
+    if (L.fp32) launch_grad_fp32(L, st);
+    else launch_grad_fp64(L, st);
 }
 
 void launch_stage(const StageLaunch& L, cudaStream_t st) {
+    if (L.order == 2) launch_gradients(L, st);
 #define CCFD_FLUX_CASE(ID) \
     case ID: launch_stage_f##ID(L, st); break;
     switch (L.flux_id) {
@@ -122,6 +129,10 @@ void launch_stage(const StageLaunch& L, cudaStream_t st) {
 
 void launch_stage_batch(const BatchLaunch& B, cudaStream_t st) {
     if (B.n_tiles <= 0) return;
+    if (B.order == 2) {
+        if (B.fp32) launch_grad_batch_fp32(B, st);
+        else launch_grad_batch_fp64(B, st);
+    }
 #define CCFD_FLUX_CASE(ID) \
     case ID: launch_stage_batch_f##ID(B, st); break;
     switch (B.flux_id) {
@@ -132,7 +143,7 @@ void launch_stage_batch(const BatchLaunch& B, cudaStream_t st) {
 #undef CCFD_FLUX_CASE
 }
 
-void launch_dt(const DevMesh& m, const Phys& P, const Ctrl* ctrl, const StepParams& sp,
+void launch_dt(const DevMesh& m, const Gas& P, const Ctrl* ctrl, const StepParams& sp,
                const double4* prim, double2* partial, int* bad_partial, cudaStream_t st) {
     k_dt<<<(m.N + 255) / 256, 256, 0, st>>>(m, P, ctrl, sp, prim, partial, bad_partial);
 }

@@ -1,18 +1,21 @@
 // Kernels of the residual-and-update path (templates shared by the
-// per-flux translation units stage_fNN.cu and by stage.cu).
+// per-flux translation units stage_fNN.cu, the gradient units gradients*.cu
+// and stage.cu).  A residual evaluation or Runge-Kutta stage is two launches:
 //
-//   k_stage  per tile (one CTA), fused: stage the primitive states of the
-//            tile, two neighbour rings and the adjacent ghost cells (ghost
-//            states at the mirrored barycentres, setBCatBarys, src/boundary.c:
-//            320-331) in shared memory; least-squares
-//            gradients with Barth-Jespersen / Venkatakrishnan limiting for the
-//            tile and ring 1 (spatialReconstruction, src/reconstruction.c:
-//            198-314); limited linear reconstruction, convective and viscous
-//            flux of every face of the tile, ghost states at boundary faces
-//            (setBCatSides, src/boundary.c:300-314; fluxCalculation,
-//            src/fluxCalculation.c:882-998); per-cell sum of the face fluxes
-//            in the reference's side order, no atomics (src/finiteVolume.c:
-//            96-120); Runge-Kutta stage update with consPrim
+//   k_grad   two threads per cell (second order only): ghost states of its
+//            boundary sides at the mirrored barycentres (setBCatBarys,
+//            src/boundary.c:320-331), least-squares gradient with
+//            Barth-Jespersen / Venkatakrishnan limiting (spatialReconstruction,
+//            src/reconstruction.c:198-314), ghost states at the boundary faces
+//            (setBCatSides, src/boundary.c:300-314).  Euler: the reconstructed
+//            states of the cell's sides go to the face records, so that k_flux
+//            streams them; Navier-Stokes: the gradients, which the viscous
+//            flux needs as well, and k_flux reconstructs.
+//   k_flux   per tile (one CTA): convective and viscous flux of every face of
+//            the tile (fluxCalculation, src/fluxCalculation.c:882-998) into
+//            shared memory; per-cell sum of the face fluxes in the
+//            reference's side order, no atomics (src/finiteVolume.c:96-120);
+//            Runge-Kutta stage update with consPrim
 //            (src/timeDiscretization.c:362-398); at the last stage the local
 //            time step of the new state and the global-residual partial sums;
 //            the CTA that finishes last reduces the partials in a fixed order
@@ -22,25 +25,31 @@
 //   k_dt / k_step_begin   calcTimeStep (src/timeDiscretization.c:249-329)
 //            for the first step of a run
 //
-// Gradients and face fluxes live only in shared memory.  Floating-point
-// operations keep the reference's operand order; the library is compiled
-// with -fmad=false, so the FP64 results equal the reference's.
+// Why two launches: a single kernel that staged the tile's states and two
+// neighbour rings in shared memory and went through gradients, faces and
+// update between barriers took 147 us per stage on the 500,000-triangle
+// double Mach reflection (HLLC, Venkatakrishnan, FP64; 108 us with FP32
+// fluxes), 344 us on 1,048,576 quads and 28 us on 8,000 quads: at most 24
+// warps per SM, ring cells computed twice, half the threads idle in the
+// second pass of each phase.  The split keeps each loop's registers low
+// enough for 28 warps, computes every gradient once and streams the face
+// states: 76, 167 and 14 us (64 us with FP32 fluxes), at 0.13 GB of DRAM
+// traffic per kernel.  Both are bound by memory latency (the scheduler
+// issues in ~45 % of its cycles) and by correctly rounded FP64 divisions.
+//
+// Floating-point operations keep the reference's operand order; the FP64
+// units are compiled with -fmad=false, so their results equal the reference's.
 #pragma once
 
 #include <cuda_runtime.h>
 
 #include <atomic>
-#include <map>
 #include <mutex>
 
 #include "kernels.cuh"
 
 namespace ccfd {
 
-// CTA shape per arithmetic type (one CTA per tile; measured): FP64 stages
-// run 384 threads, 2 CTAs per SM (gradient cells and faces of a 256-cell
-// tile in about one pass each); the FP32 kernels need half the shared
-// memory and run 256 threads, 3 CTAs per SM.
 // Dynamic shared memory limit of one kernel, raised as launches need more:
 // per device, only ever raised, and safe when host threads (the lockstep
 // implicit sets, several serving contexts) launch the same kernel at once.
@@ -62,16 +71,14 @@ struct SmemLimit {
     }
 };
 
-// Launch bounds of the stage kernels (threads, CTAs per SM: they fix the
-// registers, 80 in FP64) and the CTA size of a single-instance launch when
-// the context sets none: in FP64 256 threads, three CTAs of a 256-cell tile
-// per SM (0.147 against 0.151 ms per stage at 384 threads on the
-// 500k-triangle double Mach reflection; 320 threads: 0.169); with FP32
-// staging 128 threads on 192-cell tiles (the context's default tile size
-// in that precision), six CTAs per SM.
+// CTA shapes.  k_grad: 4 / grad_vars threads per cell, at most kGradThreads
+// per CTA.
+// k_flux: at most `threads`, `single` unless the context sets another size.
+// regs / regs_ns (viscous) / grad_regs cap the registers per thread.
+constexpr int kGradThreads = 128;
 template <typename FT> struct StageShape;
-template <> struct StageShape<double> { static constexpr int threads = 384, min_blocks = 2, single = 256; };
-template <> struct StageShape<float> { static constexpr int threads = 256, min_blocks = 3, single = 128; };
+template <> struct StageShape<double> { static constexpr int threads = 384, single = 128, regs = 72, regs_ns = 128, grad_vars = 2, grad_regs = 72; };
+template <> struct StageShape<float> { static constexpr int threads = 256, single = 128, regs = 64, regs_ns = 72, grad_vars = 2, grad_regs = 64; };
 
 __device__ __forceinline__ double stage_time(const Ctrl* ctrl, double tfix, double a_time) {
     return ctrl ? ctrl->t + a_time * ctrl->dt : tfix;
@@ -90,6 +97,59 @@ __device__ __forceinline__ double4 mk4(const double q[4]) {
 }
 __device__ __forceinline__ float4 mk4(const float q[4]) {
     return make_float4(q[0], q[1], q[2], q[3]);
+}
+
+// One 32-byte record per load / store instruction (256-bit accesses; the
+// records are 32-byte aligned): a gather then costs one request and one tag
+// lookup per sector instead of two.  ld32 is for data the kernel does not
+// write; ld32_rw keeps its place among the kernel's stores.
+__device__ __forceinline__ double4 ld32(const double4* p) {
+    double4 v;
+    asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double4 ld32_rw(const double4* p) {
+    double4 v;
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
+                 : "l"(p)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ void st32(double4* p, const double4 v) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v.x), "d"(v.y), "d"(v.z), "d"(v.w)
+                 : "memory");
+}
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
+// VPT consecutive doubles that the kernel may have written itself
+__device__ __forceinline__ void ld_rw(const double* p, double (&v)[1]) {
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v[0]) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void ld_rw(const double* p, double (&v)[2]) {
+    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "l"(p) : "memory");
+}
+// The gradients of a cell are stored variable by variable, (x0, y0, x1, y1),
+// (x2, y2, x3, y3), as the threads of the cell write them.
+__device__ __forceinline__ void ld_grad(const double4* p, double gx[4], double gy[4]) {
+    const double4 a = ld32(p), b = ld32(p + 1);
+    gx[0] = a.x; gy[0] = a.y; gx[1] = a.z; gy[1] = a.w;
+    gx[2] = b.x; gy[2] = b.y; gx[3] = b.z; gy[3] = b.w;
+}
+__device__ __forceinline__ void ld_grad(const float4* p, float gx[4], float gy[4]) {
+    asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(gx[0]), "=f"(gy[0]), "=f"(gx[1]), "=f"(gy[1]), "=f"(gx[2]), "=f"(gy[2]), "=f"(gx[3]), "=f"(gy[3])
+        : "l"(p));
+}
+// the two reconstructed states of a face
+__device__ __forceinline__ void ld_face(const double4* p, double l[4], double r[4]) {
+    ld4(ld32(p), l);
+    ld4(ld32(p + 1), r);
+}
+__device__ __forceinline__ void ld_face(const float4* p, float l[4], float r[4]) {
+    asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(l[0]), "=f"(l[1]), "=f"(l[2]), "=f"(l[3]), "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3])
+        : "l"(p));
 }
 
 // shared-memory vector types of the stage kernel: FP64 throughout, or FP32
@@ -114,75 +174,73 @@ __device__ __forceinline__ double4 to_d4(const float4& v) {
     return make_double4(v.x, v.y, v.z, v.w);
 }
 
-// Limited least-squares gradient of one cell (src/reconstruction.c:25-192,
-// 252-312).  nbr(k, qn) fetches the k-th neighbour state in side order,
-// gw(k) the side's (GP.x, GP.y, w.x, w.y), gp(k) the side's GP again for
-// the limiter.  The limiter runs side by side (each side's offset is
-// fetched once and only two of its values are live); the minimum over
-// sides and variables does not depend on the order, so the result is the
-// reference's.
-template <typename T, class Nbr, class GW, class GP>
-__device__ __forceinline__ void cell_gradient(int limiter, const T q[4], int nh, T eps2, Nbr nbr,
-                                              GW gw, GP gp, T ux[4], T uy[4]) {
-    T umin[4] = {q[0], q[1], q[2], q[3]}, umax[4] = {q[0], q[1], q[2], q[3]};
+__device__ __forceinline__ double min2(double a, double b) { return b < a ? b : a; }
+__device__ __forceinline__ double max2(double a, double b) { return b > a ? b : a; }
+__device__ __forceinline__ float min2(float a, float b) { return b < a ? b : a; }
+__device__ __forceinline__ float max2(float a, float b) { return b > a ? b : a; }
+
+// Limited least-squares gradient of NV variables of one cell (src/
+// reconstruction.c:25-192, 252-312) from their values q, the nh neighbour
+// records (nbr(k) points at the variables) and the half-side records (GP.x,
+// GP.y, w.x, w.y).  The reference evaluates the limiter of each side with the
+// largest or the smallest neighbour difference, by the sign of the
+// reconstructed difference; selecting that bound first and evaluating one
+// formula keeps warps with both signs from running it twice.  The minimum
+// over the sides does not depend on their order.
+template <int LIM, int NV, typename T, class Nbr>
+__device__ __forceinline__ void cell_gradient(const T q[NV], int nh, T eps2, Nbr nbr,
+                                              const double4* __restrict__ gw, T ux[NV], T uy[NV], T gpx[4],
+                                              T gpy[4]) {
+    T lo[NV], hi[NV];
 #pragma unroll
-    for (int v = 0; v < 4; ++v) ux[v] = uy[v] = T(0.0);
+    for (int v = 0; v < NV; ++v) {
+        lo[v] = hi[v] = q[v];
+        ux[v] = uy[v] = T(0.0);
+    }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         if (k < nh) {
-            double4 g = gw(k);
+            const double4 g = ld32(gw + k);
+            double qd[NV];
+            ld_rw(nbr(k), qd);
             const T wx = T(g.z), wy = T(g.w);
-            T qn[4];
-            nbr(k, qn);
+            gpx[k] = T(g.x);
+            gpy[k] = T(g.y);
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                T d = qn[v] - q[v];
+            for (int v = 0; v < NV; ++v) {
+                const T qn = T(qd[v]);
+                const T d = qn - q[v];
                 ux[v] += wx * d;
                 uy[v] += wy * d;
-                umin[v] = fmin(umin[v], qn[v]);
-                umax[v] = fmax(umax[v], qn[v]);
+                lo[v] = min2(lo[v], qn);
+                hi[v] = max2(hi[v], qn);
             }
         }
     }
-    T phi[4] = {T(1.0), T(1.0), T(1.0), T(1.0)};
-    T mn[4], mx[4];
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-        mn[v] = umin[v] - q[v];
-        mx[v] = umax[v] - q[v];
-    }
+    for (int v = 0; v < NV; ++v) {
+        const T mn = lo[v] - q[v], mx = hi[v] - q[v];
+        T phi = T(1.0);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        if (k < nh) {
-            T gpx, gpy;
-            gp(k, gpx, gpy);
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                T uD = ux[v] * gpx + uy[v] * gpy;
-                T pl = T(1.0);
-                if (limiter == 1) {
-                    if (uD > T(0.0)) pl = fmin(T(1.0), mx[v] / uD);
-                    else if (uD < T(0.0)) pl = fmin(T(1.0), mn[v] / uD);
-                } else {
-                    T uD2 = uD * uD;
-                    if (uD > T(0.0)) {
-                        const T mx2 = mx[v] * mx[v];
-                        pl = T(1.0) / uD * (((mx2 + eps2) * uD + T(2.0) * uD2 * mx[v]) /
-                                            (mx2 + T(2.0) * uD2 + uD * mx[v] + eps2));
-                    } else if (uD < T(0.0)) {
-                        const T mn2 = mn[v] * mn[v];
-                        pl = T(1.0) / uD * (((mn2 + eps2) * uD + T(2.0) * uD2 * mn[v]) /
-                                            (mn2 + T(2.0) * uD2 + uD * mn[v] + eps2));
+        for (int k = 0; k < 4; ++k) {
+            if (k < nh) {
+                const T uD = ux[v] * gpx[k] + uy[v] * gpy[k];
+                if (uD > T(0.0) || uD < T(0.0)) {
+                    const T m = uD > T(0.0) ? mx : mn;
+                    T pl;
+                    if constexpr (LIM == 1) {
+                        pl = m / uD;
+                    } else {
+                        const T uD2 = uD * uD, m2 = m * m;
+                        pl = T(1.0) / uD * (((m2 + eps2) * uD + T(2.0) * uD2 * m) /
+                                            (m2 + T(2.0) * uD2 + uD * m + eps2));
                     }
+                    phi = min2(phi, pl);
                 }
-                phi[v] = fmin(phi[v], pl);
             }
         }
-    }
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-        ux[v] *= phi[v];
-        uy[v] *= phi[v];
+        ux[v] *= phi;
+        uy[v] *= phi;
     }
 }
 
@@ -191,7 +249,7 @@ __device__ __forceinline__ void cell_gradient(int limiter, const T q[4], int nh,
 // (src/fluxCalculation.c:885-996).  q0 / q1 are the cell-centre states and
 // g0x..g1y the cell gradients (Navier-Stokes only).
 template <int FLUX, int NS, typename T>
-__device__ __forceinline__ void face_flux(const Phys& P, T nx, T ny, T len, const T L[4], const T R[4],
+__device__ __forceinline__ void face_flux(const Gas& P, T nx, T ny, T len, const T L[4], const T R[4],
                                           const T q0[4], const T q1[4], const T g0x[4],
                                           const T g0y[4], const T g1x[4], const T g1y[4], double4 bbd,
                                           T F[4], unsigned* flags) {
@@ -242,14 +300,27 @@ static __device__ __noinline__ double4 ghost_bary(const int* __restrict__ gbc, c
 
 // ghost state at a boundary face from the reconstructed interior face state
 static __device__ __noinline__ double4 ghost_face(const int* __restrict__ gbc, const double4* __restrict__ ggn,
-                                           const double4* __restrict__ gml, const Phys* __restrict__ Pg,
+                                           const double2* __restrict__ mid, const Phys* __restrict__ Pg,
                                            int g, double time, double4 Lv, unsigned* flags) {
     const Phys& P = *Pg;
-    double4 gn = ggn[g], ml = gml[g];
-    double x[2] = {ml.x, ml.y};
+    const double4 gn = ggn[g];
+    const double2 xm = mid[g];
+    double x[2] = {xm.x, xm.y};
     double Lq[4] = {Lv.x, Lv.y, Lv.z, Lv.w}, R[4];
     boundary_state(P, P.bc[gbc[g]], gn.z, gn.w, time, Lq, R, x, flags);
     return make_double4(R[0], R[1], R[2], R[3]);
+}
+
+// the same, noting the interior pressure at the face for the wing
+// coefficients
+__device__ __forceinline__ double4 boundary_face(const StageLaunch& L, int g, double time, double4 q) {
+    if (L.ghost_pface) L.ghost_pface[g] = q.w;
+    return ghost_face(L.ghosts.bc, L.ghosts.gn, L.ghosts.mid, L.phys_g, g, time, q, L.flags);
+}
+
+// owner and neighbour cell (-1-g: ghost g) in a face record's last word
+__device__ __forceinline__ int2 face_cells(const double4& nl) {
+    return make_int2(__double2loint(nl.w), __double2hiint(nl.w));
 }
 
 template <int NV>
@@ -305,10 +376,41 @@ __device__ __forceinline__ void block_min2(double a, double b, int bad, double2*
     }
 }
 
+// Tile reduction of the last stage: per-thread sums of the four residual
+// partials and the minima of the time steps.  The values pass through shared
+// memory (red, 6 * blockDim.x doubles) so that one warp finishes one value:
+// five shuffle steps per value and CTA instead of per value and warp.
+__device__ __forceinline__ void tile_reduce(const double r[4], double dconv, double dvisc, int bad, bool visc,
+                                            double* red, double* res_out, double2* dt_out, int* bad_out) {
+    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31;
+    __syncthreads();  // red may overlay data other threads still read
+#pragma unroll
+    for (int v = 0; v < 4; ++v) red[v * nthr + tid] = r[v];
+    red[4 * nthr + tid] = dconv;
+    if (visc) red[5 * nthr + tid] = dvisc;
+    bad = __syncthreads_or(bad);
+    for (int v = tid >> 5; v < 6; v += nthr >> 5) {
+        double x = v < 4 ? 0.0 : 1e150;
+        if (v < 5 || visc)
+            for (int i = lane; i < nthr; i += 32) x = v < 4 ? x + red[v * nthr + i] : fmin(x, red[v * nthr + i]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double y = __shfl_down_sync(0xffffffffu, x, o);
+            x = v < 4 ? x + y : fmin(x, y);
+        }
+        if (lane == 0) {
+            if (v < 4) res_out[v] = x;
+            else if (v == 4) dt_out->x = x;
+            else dt_out->y = x;
+        }
+    }
+    if (tid == 0) *bad_out = bad;
+}
+
 // local convective / viscous time step of one cell (calcTimeStep,
 // src/timeDiscretization.c:253-308) at CFL number cfl; returns false if not
 // finite
-__device__ __forceinline__ bool local_dt(const Phys& P, const StepParams& sp, double cfl, double dfl,
+__device__ __forceinline__ bool local_dt(const Gas& P, const StepParams& sp, double cfl, double dfl,
                                          const double q[4], double4 geo, double* dc, double* dv) {
     double a = sqrt(P.gam * q[3] / q[0]);
     *dv = 1e150;
@@ -345,6 +447,8 @@ __device__ __forceinline__ void finish_dt(Ctrl* ctrl, const StepParams& sp, doub
     ctrl->dt = dt;
 }
 
+constexpr int kWallChunk = 256;  // wall faces per pass of the wing-coefficient sums
+
 // End of a step, executed by one whole block: global residual (fixed-order
 // reduction of the per-tile partials), wing coefficients, t += dt, the stop
 // tests of timeDisc (src/timeDiscretization.c:609-731), the CFL number of
@@ -363,15 +467,66 @@ __device__ __forceinline__ void step_end_block(Ctrl* ctrl, const StepParams& sp,
     double r[4] = {0.0, 0.0, 0.0, 0.0};
     double a = 1e150, b = 1e150;
     int bad = 0;
-    for (int i = tid; i < nres; i += blockDim.x)
+    // each thread adds its partials in index order; kLd loads are issued at
+    // a time, so that the sum over thousands of tiles is not one L2 round
+    // trip per partial
+    constexpr int kLd = 8;
+    const int nthr = blockDim.x;
+    for (int i0 = tid; i0 < nres; i0 += kLd * nthr) {
+        double2 p[kLd][2];
 #pragma unroll
-        for (int v = 0; v < 4; ++v) r[v] += __ldcg(&res_partial[4 * i + v]);
-    for (int i = tid; i < ndt; i += blockDim.x) {
-        double2 d = __ldcg(&dt_partial[i]);
-        a = fmin(a, d.x);
-        b = fmin(b, d.y);
-        bad |= __ldcg(&dt_bad[i]);
+        for (int j = 0; j < kLd; ++j) {
+            const int i = i0 + j * nthr;
+            const double2* src = reinterpret_cast<const double2*>(res_partial + 4 * (size_t)(i < nres ? i : i0));
+            p[j][0] = __ldcg(src);
+            p[j][1] = __ldcg(src + 1);
+        }
+#pragma unroll
+        for (int j = 0; j < kLd; ++j)
+            if (i0 + j * nthr < nres) {
+                r[0] += p[j][0].x;
+                r[1] += p[j][0].y;
+                r[2] += p[j][1].x;
+                r[3] += p[j][1].y;
+            }
     }
+    for (int i0 = tid; i0 < ndt; i0 += kLd * nthr) {
+        double2 p[kLd];
+        int e[kLd];
+#pragma unroll
+        for (int j = 0; j < kLd; ++j) {
+            const int i = i0 + j * nthr < ndt ? i0 + j * nthr : i0;
+            p[j] = __ldcg(&dt_partial[i]);
+            e[j] = __ldcg(&dt_bad[i]);
+        }
+#pragma unroll
+        for (int j = 0; j < kLd; ++j) {
+            a = fmin(a, p[j].x);
+            b = fmin(b, p[j].y);
+            bad |= e[j];
+        }
+    }
+    // wing coefficients: the terms by the whole block, their sums by one
+    // thread in the reference's order
+    __shared__ double s_wl[2][kWallChunk];
+    double cl = 0.0, cd = 0.0;
+    if (sp.calc_wing)
+        for (int k0 = 0; k0 < sp.n_wall; k0 += kWallChunk) {
+            const int n = min(kWallChunk, sp.n_wall - k0);
+            for (int k = tid; k < n; k += nthr) {
+                const double p0 = __ldcg(&ghost_pface[wall_ghost[k0 + k]]);
+                const double* nl = wall_nl + 3 * (size_t)(k0 + k);
+                s_wl[0][k] = nl[1] * p0 * nl[2];
+                s_wl[1][k] = nl[0] * p0 * nl[2];
+            }
+            __syncthreads();
+            if (tid == 0)
+                for (int k = 0; k < n; ++k) {
+                    cl += s_wl[0][k];
+                    cd += s_wl[1][k];
+                }
+            __syncthreads();
+        }
     block_sum<4>(r, s_res);
     block_min2(a, b, bad, &s_dt, &s_bad);
     __syncthreads();
@@ -386,13 +541,6 @@ __device__ __forceinline__ void step_end_block(Ctrl* ctrl, const StepParams& sp,
     ctrl->iter = iter;
     if (sp.calc_wing) {
         double cl_old = ctrl->cl, cd_old = ctrl->cd;
-        double cl = 0.0, cd = 0.0;
-        for (int k = 0; k < sp.n_wall; ++k) {
-            double p0 = __ldcg(&ghost_pface[wall_ghost[k]]);
-            double wnx = wall_nl[3 * k], wny = wall_nl[3 * k + 1], wl = wall_nl[3 * k + 2];
-            cl += wny * p0 * wl;
-            cd += wnx * p0 * wl;
-        }
         cl *= sp.q_inf_lq;
         cd *= sp.q_inf_lq;
         ctrl->cl = cl * sp.cos_a - cd * sp.sin_a;
@@ -477,206 +625,271 @@ __device__ __forceinline__ void step_end_block(Ctrl* ctrl, const StepParams& sp,
     if (with_dt) finish_dt(ctrl, sp, s_dt.x, s_dt.y, s_bad);
 }
 
-// fused residual evaluation (+ RK stage) of tile t by one CTA; FT is the
-// arithmetic type of the reconstruction and the face fluxes
-template <int FLUX, int ORDER, int NS, typename FT>
-__device__ __forceinline__ void stage_body(const StageLaunch& L, const int t) {
+// limited reconstruction of tile t's cells and the ghost states of their
+// boundary sides; 4 / NV consecutive threads treat one cell, thread `part`
+// its variables NV part ... (a fraction of the registers of one thread per
+// cell, so more warps hide the gathers).  The boundary code runs in loops of
+// its own over the tile's ghosts, before and after the cells: called from the
+// cell loop its registers spilled the loop's.
+template <int LIM, int NS, typename FT>
+__device__ __forceinline__ void grad_body(const StageLaunch& L, const int t) {
     using V4 = typename Vec<FT>::v4;
-    using V2 = typename Vec<FT>::v2;
-    extern __shared__ double4 smem[];
+    constexpr int NV = StageShape<FT>::grad_vars, G = 4 / NV;
     const DevMesh& m = L.mesh;
-    const TileDev& T = L.tiles;
-    const Phys& P = L.phys;
-    const int tid = threadIdx.x;
-    // CTA size: the precision's default shape, or a smaller one chosen for the
-    // context (the launch bounds fix the registers; work is strided by it)
-    const int nthr = blockDim.x;
-    const int4 cnt = T.counts[t];
-    const int nT = cnt.x, nG = cnt.y, nEc = cnt.z, nE = cnt.w;
-    const int e0 = T.e_off[t];
-    // the tile's own cells are consecutive device cells (staged entries
-    // 0..nT-1): their indices need no lookup
-    const int d_first = T.e_ref[e0];
-    const double time = stage_time(L.ctrl, L.tfix, L.a_time);
-    V4* ps = reinterpret_cast<V4*>(smem);             // [max_e] states
-    V4* gs = ps + T.max_e;                            // [2 max_g] gradients
-    V2* hgp = reinterpret_cast<V2*>(gs + 2 * T.max_g);  // [max_hs] GP
-    V4* fs = reinterpret_cast<V4*>(hgp + T.max_hs + (T.max_hs & 1));  // [max_f]
-
-    // source term of the tile's cells (calcSource), evaluated first, while
-    // few registers are live, into a per-cell buffer that the same thread
-    // reads back in D (same cell-to-thread mapping)
-    if (m.cell_src)
-        for (int i = tid; i < nT; i += nthr) {
-            const int d = d_first + i;
-            m.src_buf[d] = cell_source(P, m.hs_gw, m.hs_off[d], m.hs_off[d + 1], m.cell_src[d],
-                                       m.cell_geo[d].x, time);
-        }
-
-    // A: stage the states of the tile and its rings; ghost cells get the
-    // boundary state at their mirrored barycentre (second order only: the
-    // reference sets ghost cell states in its second-order reconstruction
-    // and leaves them zero otherwise)
-    for (int e = tid; e < nEc; e += nthr)
-        ps[e] = cvt4<FT>(L.prim_in[e < nT ? d_first + e : T.e_ref[e0 + e]]);
-    for (int e = nEc + tid; e < nE; e += nthr) {
-        int g = -1 - T.e_ref[e0 + e];
-        double4 gq = make_double4(0.0, 0.0, 0.0, 0.0);
-        if (ORDER == 2)
-            gq = ghost_bary(L.ghosts.bc, L.ghosts.gn, L.phys_g, g, time, L.prim_in[L.ghosts.cell[g]],
-                            L.flags);
-        ps[e] = cvt4<FT>(gq);
-    }
-    __syncthreads();
-
-    // B: limited gradients of the tile and ring-1 cells
-    const int hb = T.hs_off[t], gb = T.gl_off[t];
-    if (ORDER == 2) {
-        for (int i = tid; i < nG; i += nthr) {
-            int d = i < nT ? d_first + i : T.e_ref[e0 + i];
-            int h0 = m.hs_off[d], nh = m.hs_off[d + 1] - h0;
-            int lo = T.hs_loc[gb + i];
-            FT q[4], ux[4], uy[4];
-            ld4(ps[i], q);
-            FT eps2 = L.limiter == 2 ? FT(m.venk_eps2[d]) : FT(0.0);
-            auto nbr = [&](int k, FT qn[4]) { ld4(ps[T.hs_nbl[hb + lo + k]], qn); };
-            auto gw = [&](int k) {
-                double4 g = m.hs_gw[h0 + k];
-                hgp[lo + k] = cvt2<FT>(g.x, g.y);
-                return g;
-            };
-            auto gp = [&](int k, FT& x, FT& y) {
-                const V2 g = hgp[lo + k];
-                x = g.x;
-                y = g.y;
-            };
-            cell_gradient<FT>(L.limiter, q, nh, eps2, nbr, gw, gp, ux, uy);
-            gs[2 * i] = mk4(ux);
-            gs[2 * i + 1] = mk4(uy);
+    const int2 gr = L.tiles.g_rng[t];
+    if (gr.y > 0) {
+        const double time = stage_time(L.ctrl, L.tfix, L.a_time);
+        for (int i = threadIdx.x; i < gr.y; i += blockDim.x) {
+            const int4 e = L.tiles.ghost[gr.x + i];
+            L.ghosts.state[e.x] =
+                ghost_bary(L.ghosts.bc, L.ghosts.gn, L.phys_g, e.x, time, L.prim_in[e.y], L.flags);
         }
         __syncthreads();
     }
-
-    // C: fluxes of the tile's faces (interior faces, then boundary faces)
-    const int f0 = T.f_off[t], nF = T.f_off[t + 1] - f0;
-    for (int j = tid; j < nF; j += nthr) {
-        int fid = T.f_id[f0 + j];
-        int lr = T.f_lr[f0 + j];
-        int il = lr & 0xffff, ir = lr >> 16;
-        FT q0[4], q1[4], Lf[4], Rf[4];
-        FT g0x[4] = {0, 0, 0, 0}, g0y[4] = {0, 0, 0, 0}, g1x[4] = {0, 0, 0, 0}, g1y[4] = {0, 0, 0, 0};
-        ld4(ps[il], q0);
-        ld4(ps[ir], q1);
-        int hh = T.f_hs[f0 + j];
-        if (ORDER == 2) {
-            V2 gpl = hgp[hh & 0xffff];
-            ld4(gs[2 * il], g0x);
-            ld4(gs[2 * il + 1], g0y);
+    const int v0 = NV * (int)(threadIdx.x % G);
+    const int d_end = min(m.N, (t + 1) * L.tiles.cells);
+    for (int d = t * L.tiles.cells + (int)(threadIdx.x / G); d < d_end; d += blockDim.x / G) {
+        const int4 nb = m.nb4[d];
+        const int h0 = m.hs_off[d];
+        const int4 sl = NS ? make_int4(0, 0, 0, 0) : m.slot4[d];
+        const FT eps2 = LIM == 2 ? FT(m.venk_eps2[d]) : FT(0.0);
+        double qd[NV];
+        ld_rw(reinterpret_cast<const double*>(L.prim_in + d) + v0, qd);
+        const int nbv[4] = {nb.x, nb.y, nb.z, nb.w};
+        auto nbr = [&](int k) {
+            return reinterpret_cast<const double*>(nbv[k] < 0 ? L.ghosts.state + (-1 - nbv[k]) : L.prim_in + nbv[k]) +
+                   v0;
+        };
+        const int nh = nb.w == kNoSide ? 3 : 4;
+        FT q[NV], ux[NV], uy[NV], gpx[4], gpy[4];
 #pragma unroll
-            for (int v = 0; v < 4; ++v) Lf[v] = q0[v] + gpl.x * g0x[v] + gpl.y * g0y[v];
-        } else {
+        for (int v = 0; v < NV; ++v) q[v] = FT(qd[v]);
+        cell_gradient<LIM, NV, FT>(q, nh, eps2, nbr, m.hs_gw + h0, ux, uy, gpx, gpy);
+        if (NS) {
+            FT* g = reinterpret_cast<FT*>(L.grad) + 8 * (size_t)d + 2 * v0;
 #pragma unroll
-            for (int v = 0; v < 4; ++v) Lf[v] = q0[v];
+            for (int v = 0; v < NV; ++v) {
+                g[2 * v] = ux[v];
+                g[2 * v + 1] = uy[v];
+            }
         }
-        FT nx, ny, len;
-        double4 bb = make_double4(0, 0, 1, 0);
-        if (fid >= 0) {
-            if (ORDER == 2) {
-                V2 gpr = hgp[hh >> 16];
-                ld4(gs[2 * ir], g1x);
-                ld4(gs[2 * ir + 1], g1y);
+        if (L.grad_out) {
+            double* g = reinterpret_cast<double*>(L.grad_out) + 8 * (size_t)d + 2 * v0;
 #pragma unroll
-                for (int v = 0; v < 4; ++v) Rf[v] = q1[v] + gpr.x * g1x[v] + gpr.y * g1y[v];
+            for (int v = 0; v < NV; ++v) {
+                g[2 * v] = double(ux[v]);
+                g[2 * v + 1] = double(uy[v]);
+            }
+        }
+        // reconstructed states of the sides: Euler into the face records,
+        // Navier-Stokes those of boundary sides only
+        const int slv[4] = {sl.x, sl.y, sl.z, sl.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (k < nh && (!NS || nbv[k] < 0)) {
+                FT f[NV];
+#pragma unroll
+                for (int v = 0; v < NV; ++v) f[v] = q[v] + gpx[k] * ux[v] + gpy[k] * uy[v];
+                if (NS) {
+                    double* o = reinterpret_cast<double*>(L.ghosts.face + (-1 - nbv[k])) + v0;
+#pragma unroll
+                    for (int v = 0; v < NV; ++v) o[v] = double(f[v]);
+                } else {
+                    FT* o = reinterpret_cast<FT*>(L.fstate) + 4 * (size_t)slv[k] + v0;
+                    if constexpr (NV == 2) *reinterpret_cast<typename Vec<FT>::v2*>(o) = typename Vec<FT>::v2{f[0], f[1]};
+                    else *o = f[0];
+                }
+            }
+        }
+    }
+    if (gr.y > 0) {
+        __syncthreads();
+        const double time = stage_time(L.ctrl, L.tfix, L.a_time);
+        for (int i = threadIdx.x; i < gr.y; i += blockDim.x) {
+            const int4 e = L.tiles.ghost[gr.x + i];
+            V4* const fst = reinterpret_cast<V4*>(L.fstate) + e.z;
+            const double4 q = NS ? L.ghosts.face[e.x] : to_d4(fst[0]);
+            const double4 R = boundary_face(L, e.x, time, q);
+            if (NS) L.ghosts.face[e.x] = R;
+            else fst[1] = cvt4<FT>(R);
+        }
+    }
+}
+
+// fluxes of the faces of tile t, residual (+ RK stage) of its cells; FT is
+// the arithmetic type of the reconstruction and the face fluxes
+template <int FLUX, int ORDER, int NS, typename FT>
+__device__ __forceinline__ void flux_body(const StageLaunch& L, const int t) {
+    using V4 = typename Vec<FT>::v4;
+    extern __shared__ double4 smem[];
+    using V2 = typename Vec<FT>::v2;
+    // face fluxes in two planes of half records: consecutive threads then
+    // access consecutive 16 (8) bytes, without bank conflicts
+    V2* const fa = reinterpret_cast<V2*>(smem);
+    V2* const fb = fa + L.tiles.max_f;
+    auto put = [&](int j, const FT q[4]) {
+        fa[j] = V2{q[0], q[1]};
+        fb[j] = V2{q[2], q[3]};
+    };
+    auto get = [&](int j, FT q[4]) {
+        const V2 a = fa[j], b = fb[j];
+        q[0] = a.x; q[1] = a.y; q[2] = b.x; q[3] = b.y;
+    };
+    const DevMesh& m = L.mesh;
+    const TileDev& T = L.tiles;
+    const Gas& P = L.gas;
+    const int tid = threadIdx.x, nthr = blockDim.x;
+    const int4 rng = T.rng[t];
+    const int nO = rng.y, nF = rng.y + rng.w;
+    const int d0 = t * T.cells, d_end = min(m.N, d0 + T.cells);
+    auto face_id = [&](int j) { return j < nO ? rng.x + j : T.border[rng.z + j - nO]; };
+    // what the update of this thread's first cell will read
+    if (d0 + tid < d_end) {
+        prefetch_l1(T.u_code + d0 + tid);
+        prefetch_l1(m.area_q + d0 + tid);
+        if (L.mode == 1) prefetch_l1(L.cons0 + d0 + tid);
+    }
+
+    // source term of the tile's cells (calcSource), evaluated first, while
+    // few registers are live, into a per-cell buffer that the same thread
+    // reads back below (same cell-to-thread mapping)
+    if (m.cell_src) {
+        const double time = stage_time(L.ctrl, L.tfix, L.a_time);
+        for (int d = d0 + tid; d < d_end; d += nthr)
+            m.src_buf[d] = cell_source(*L.phys_g, m.hs_gw, m.hs_off[d], m.hs_off[d + 1], m.cell_src[d],
+                                       m.cell_geo[d].x, time);
+    }
+
+    if (ORDER == 1) {
+        // first order: the ghost states of the boundary faces, from the cell
+        // states (in second order k_grad has written them)
+        const int2 gr = T.g_rng[t];
+        if (gr.y > 0) {
+            const double time = stage_time(L.ctrl, L.tfix, L.a_time);
+            for (int i = tid; i < gr.y; i += nthr) {
+                const int4 e = T.ghost[gr.x + i];
+                L.ghosts.face[e.x] = boundary_face(L, e.x, time, to_d4(cvt4<FT>(L.prim_in[e.y])));
+            }
+            __syncthreads();
+        }
+    }
+
+    // fluxes of the tile's faces
+    int id_next = tid < nF ? face_id(tid) : 0;
+    for (int j = tid; j < nF; j += nthr) {
+        const int id = id_next;
+        if (j + nthr < nF) id_next = face_id(j + nthr);
+        const double4 nl = ld32(T.f_nl + id);
+        FT q0[4] = {0, 0, 0, 0}, q1[4] = {0, 0, 0, 0}, Lf[4], Rf[4];
+        FT g0x[4] = {0, 0, 0, 0}, g0y[4] = {0, 0, 0, 0}, g1x[4] = {0, 0, 0, 0}, g1y[4] = {0, 0, 0, 0};
+        double4 bb = make_double4(0, 0, 1, 0);
+        if (ORDER == 2 && !NS) {
+            ld_face(reinterpret_cast<const V4*>(L.fstate) + 2 * (size_t)id, Lf, Rf);
+        } else {
+            // ghost cells: a state at the mirrored barycentre in second
+            // order (zero in first order, as in the reference), no gradient
+            const int2 lr = face_cells(nl);
+            const bool inner = lr.y >= 0;
+            if (NS) bb = ld32(T.f_bb + id);
+            ld4(cvt4<FT>(ld32(L.prim_in + lr.x)), q0);
+            if (inner) ld4(cvt4<FT>(ld32(L.prim_in + lr.y)), q1);
+            else if (ORDER == 2) ld4(cvt4<FT>(ld32(L.ghosts.state + (-1 - lr.y))), q1);
+            if (ORDER == 2) {
+                const V4* grad = reinterpret_cast<const V4*>(L.grad);
+                const double4 gp = ld32(T.f_gp + id);
+                const FT pxl = FT(gp.x), pyl = FT(gp.y), pxr = FT(gp.z), pyr = FT(gp.w);
+                ld_grad(grad + 2 * (size_t)lr.x, g0x, g0y);
+#pragma unroll
+                for (int v = 0; v < 4; ++v) Lf[v] = q0[v] + pxl * g0x[v] + pyl * g0y[v];
+                if (inner) {
+                    ld_grad(grad + 2 * (size_t)lr.y, g1x, g1y);
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) Rf[v] = q1[v] + pxr * g1x[v] + pyr * g1y[v];
+                }
             } else {
 #pragma unroll
-                for (int v = 0; v < 4; ++v) Rf[v] = q1[v];
+                for (int v = 0; v < 4; ++v) {
+                    Lf[v] = q0[v];
+                    Rf[v] = q1[v];
+                }
             }
-            double4 nl = m.face_nl[fid];
-            nx = FT(nl.x); ny = FT(nl.y); len = FT(nl.z);
-            if (NS) bb = m.face_bb[fid];
-        } else {
-            int g = -1 - fid;
-            double4 Rd = ghost_face(L.ghosts.bc, L.ghosts.gn, L.ghosts.ml, L.phys_g, g, time,
-                                    to_d4(mk4(Lf)), L.flags);
-            ld4(cvt4<FT>(Rd), Rf);
-            if (L.ghost_pface) L.ghost_pface[g] = double(Lf[3]);
-            double4 gn = L.ghosts.gn[g];
-            nx = FT(gn.z); ny = FT(gn.w); len = FT(L.ghosts.ml[g].z);
-            if (NS) bb = L.ghosts.bb[g];
+            if (!inner) ld4(cvt4<FT>(ld32_rw(L.ghosts.face + (-1 - lr.y))), Rf);
         }
         FT F[4];
-        face_flux<FLUX, NS, FT>(P, nx, ny, len, Lf, Rf, q0, q1, g0x, g0y, g1x, g1y, bb, F, L.flags);
-        fs[j] = mk4(F);
+        face_flux<FLUX, NS, FT>(P, FT(nl.x), FT(nl.y), FT(nl.z), Lf, Rf, q0, q1, g0x, g0y, g1x, g1y, bb, F, L.flags);
+        put(j, F);
     }
     __syncthreads();
 
-    // D: per-cell flux sum in side order, update
+    // per-cell flux sum in side order, update
     double r[4] = {0, 0, 0, 0};
     double dconv = 1e150, dvisc = 1e150;
     int bad = 0;
     const bool rk = L.mode == 1;
-    for (int i = tid; i < nT; i += nthr) {
-        int d = d_first + i;
-        int h0 = m.hs_off[d], h1 = m.hs_off[d + 1];
+    for (int d = d0 + tid; d < d_end; d += nthr) {
+        const ushort4 code = T.u_code[d];
+        const unsigned cv[4] = {code.x, code.y, code.z, code.w};
         double s[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int h = h0; h < h1; ++h) {
-            int code = T.u_code[h];
-            FT F[4];
-            ld4(fs[code >> 1], F);
-            if (code & 1) {
 #pragma unroll
-                for (int v = 0; v < 4; ++v) s[v] += -double(F[v]);
-            } else {
+        for (int k = 0; k < 4; ++k) {
+            if (cv[k] != 0xffffu) {
+                FT F[4];
+                get(cv[k] >> 1, F);
+                const bool neg = cv[k] & 1u;
 #pragma unroll
-                for (int v = 0; v < 4; ++v) s[v] += double(F[v]);
+                for (int v = 0; v < 4; ++v) s[v] += neg ? -double(F[v]) : double(F[v]);
             }
         }
-        double4 geo = m.cell_geo[d];
         const double4 sv = m.cell_src ? m.src_buf[d] : make_double4(0.0, 0.0, 0.0, 0.0);
         const double src[4] = {sv.x, sv.y, sv.z, sv.w};
+        const double aq = m.area_q[d];
         double ut[4];
 #pragma unroll
-        for (int v = 0; v < 4; ++v) ut[v] = (src[v] - s[v]) * geo.y;
-        if (L.u_t) L.u_t[d] = mk4(ut);
-        if (!rk && L.grad_out) {
-            L.grad_out[2 * d] = ORDER == 2 ? to_d4(gs[2 * i]) : make_double4(0, 0, 0, 0);
-            L.grad_out[2 * d + 1] = ORDER == 2 ? to_d4(gs[2 * i + 1]) : make_double4(0, 0, 0, 0);
-        }
+        for (int v = 0; v < 4; ++v) ut[v] = (src[v] - s[v]) * aq;
+        if (L.u_t) st32(L.u_t + d, mk4(ut));
         if (rk) {
             double c0[4], cn[4], pn[4];
-            ld4(L.cons0[d], c0);
+            ld4(ld32_rw(L.cons0 + d), c0);
             double adt = L.rk * L.ctrl->dt;
 #pragma unroll
             for (int v = 0; v < 4; ++v) cn[v] = c0[v] + adt * ut[v];
             cons_prim(P.gam1, cn, pn);
-            L.prim_out[d] = mk4(pn);
+            st32(L.prim_out + d, mk4(pn));
             if (L.last_stage) {
-                L.cons0[d] = mk4(cn);
+                st32(L.cons0 + d, mk4(cn));
                 double a, b;
-                if (!local_dt(P, L.sp, L.sp.cfl, L.sp.dfl, pn, geo, &a, &b)) bad = 1;
+                if (!local_dt(P, L.sp, L.sp.cfl, L.sp.dfl, pn, m.cell_geo[d], &a, &b)) bad = 1;
                 else {
                     dconv = fmin(dconv, a);
                     dvisc = fmin(dvisc, b);
                 }
             }
         }
+        if (L.res_partial) {
+            const double area = m.cell_geo[d].x;
 #pragma unroll
-        for (int v = 0; v < 4; ++v) r[v] += geo.x * ut[v] * ut[v];
+            for (int v = 0; v < 4; ++v) r[v] += area * ut[v] * ut[v];
+        }
     }
-    if (L.res_partial) {
+    if (L.dt_partial) {
+        tile_reduce(r, dconv, dvisc, bad, L.sp.visc, reinterpret_cast<double*>(smem), &L.res_partial[4 * t],
+                    &L.dt_partial[t], &L.dt_bad[t]);
+    } else if (L.res_partial) {
         double out[4];
         block_sum<4>(r, out);
         if (tid == 0)
 #pragma unroll
             for (int v = 0; v < 4; ++v) L.res_partial[4 * t + v] = out[v];
     }
-    if (L.dt_partial) block_min2(dconv, dvisc, bad, &L.dt_partial[t], &L.dt_bad[t]);
     if (rk && L.last_stage) {
-        // the CTA that finishes last closes the step
+        // the CTA that finishes last closes the step (one thread's fence
+        // covers what the CTA wrote before the barrier)
         __shared__ int s_last;
-        __threadfence();
         __syncthreads();
-        if (tid == 0) s_last = atomicAdd(L.ticket, 1u) == (unsigned)(T.n_tiles - 1);
+        if (tid == 0) {
+            __threadfence();
+            s_last = atomicAdd(L.ticket, 1u) == (unsigned)(T.n_tiles - 1);
+        }
         __syncthreads();
         if (s_last) {
             __threadfence();
@@ -691,116 +904,101 @@ __device__ __forceinline__ void stage_body(const StageLaunch& L, const int t) {
     }
 }
 
-
 // one instance: one tile per CTA, launch parameters in the parameter space
-template <int FLUX, int ORDER, int NS, typename FT>
-__global__ void __launch_bounds__(StageShape<FT>::threads, StageShape<FT>::min_blocks) k_stage(StageLaunch L) {
+template <int LIM, int NS, typename FT>
+__global__ void __maxnreg__(StageShape<FT>::grad_regs) k_grad(const __grid_constant__ StageLaunch L) {
     if (inactive(L.ctrl)) return;
-    stage_body<FLUX, ORDER, NS, FT>(L, blockIdx.x);
+    grad_body<LIM, NS, FT>(L, blockIdx.x);
 }
 
-// Many instances in one persistent launch over their concatenated tiles:
-// each CTA claims the next entry of the tile map from a counter (entry b is
-// tile tmap[b].y of instance tmap[b].x) until none is left, so uneven
-// instances share one grid sized to the device, and CTAs that cannot start
-// at once (SMs held by other work of the device) leave their share to the
-// running ones instead of holding the launch back.  ctr[0] is the next
-// entry, ctr[1] the CTAs done; the last CTA to finish resets both for the
-// next launch on the stream.  An RK stage takes the instance's launch
-// record for the stage and the buffer parity in its control block
-// (Ls[inst][par][stage]); a residual evaluation (stride 1) takes Ls[inst]
-// and is skipped while *skip is nonzero.
 template <int FLUX, int ORDER, int NS, typename FT>
-__global__ void __launch_bounds__(StageShape<FT>::threads, StageShape<FT>::min_blocks)
-    k_stage_batch(const StageLaunch* __restrict__ Ls, const int2* __restrict__ tmap, int n_tiles, int rk_mode,
-                  int stage, int* __restrict__ ctr) {
-    // The member's launch record goes to shared memory.  In RK mode the
-    // records of both buffer parities are copied while one thread reads the
-    // member's control block, so resolving the record costs one round trip
-    // after the tile map instead of a chain of dependent loads.
+__global__ void __maxnreg__(NS ? StageShape<FT>::regs_ns : StageShape<FT>::regs) k_flux(const __grid_constant__ StageLaunch L) {
+    if (inactive(L.ctrl)) return;
+    // last tile first: what k_grad wrote last is still in L2, and the next
+    // k_grad starts with the states written last here
+    flux_body<FLUX, ORDER, NS, FT>(L, L.tiles.n_tiles - 1 - (int)blockIdx.x);
+}
+
+// Many instances in one launch over their concatenated tiles: entry b of the
+// tile map names the instance, its tile and the word that says whether the
+// instance steps.  The CTA copies the instance's record to shared memory
+// while one thread reads that word (one round trip after the map entry); an
+// RK stage then takes its state buffers from the parity in the control block
+// and its coefficients from the instance's table.  False: nothing to do.
+__device__ __forceinline__ bool batch_record(const StageLaunch* __restrict__ recs, const int4 e, int rk_mode,
+                                             int stage, StageLaunch& L) {
     static_assert(sizeof(StageLaunch) % 16 == 0, "launch record copied in 16-byte words");
     constexpr int W = (int)(sizeof(StageLaunch) / 16);
-    __shared__ int4 s_rec[2 * W];
-    __shared__ int s_go, s_sel, s_b;
-    for (;;) {
-        __syncthreads();  // the previous entry's record is no longer read
-        if (threadIdx.x == 0) s_b = atomicAdd(&ctr[0], 1);
-        __syncthreads();
-        const int b = s_b;
-        if (b >= n_tiles) break;
-        const int2 tm = tmap[b];
+    __shared__ int s_go, s_par;
+    const int4* src = reinterpret_cast<const int4*>(recs + e.x);
+    for (int k = threadIdx.x; k < W; k += blockDim.x) reinterpret_cast<int4*>(&L)[k] = src[k];
+    if (threadIdx.x == 0) {
+        const unsigned long long w = ((unsigned long long)(unsigned)e.w << 32) | (unsigned)e.z;
         if (rk_mode) {
-            const StageLaunch* rec = Ls + (size_t)tm.x * 2 * kBatchStages;
-            const int4* a = reinterpret_cast<const int4*>(rec + stage);
-            const int4* c = reinterpret_cast<const int4*>(rec + kBatchStages + stage);
-            for (int k = threadIdx.x; k < 2 * W; k += blockDim.x) s_rec[k] = k < W ? a[k] : c[k - W];
-            if (threadIdx.x == 0) {
-                const Ctrl* cb = rec[0].ctrl;
-                s_go = cb->active;
-                s_sel = cb->par;
-            }
+            const Ctrl* cb = reinterpret_cast<const Ctrl*>(w);
+            s_go = cb->active;
+            s_par = cb->par;
         } else {
-            const int4* a = reinterpret_cast<const int4*>(Ls + tm.x);
-            for (int k = threadIdx.x; k < W; k += blockDim.x) s_rec[k] = a[k];
-            if (threadIdx.x == 0) {
-                const int* skip = Ls[tm.x].skip;
-                s_go = !(skip && *skip);
-                s_sel = 0;
+            const int* skip = reinterpret_cast<const int*>(w);
+            s_go = !(skip && *skip);
+        }
+    }
+    __syncthreads();
+    if (!s_go) return false;
+    if (rk_mode) {
+        if (stage >= L.sp.nrk) return false;
+        __syncthreads();  // every thread has read nrk and the go word
+        if (threadIdx.x == 0) {
+            const int in = s_par ^ (stage & 1);
+            L.prim_in = L.prim_buf[in];
+            L.prim_out = L.prim_buf[in ^ 1];
+            L.a_time = L.sp.rk[stage];
+            L.rk = L.sp.rk[stage + 1];
+            L.last_stage = stage == L.sp.nrk - 1;
+            if (!L.last_stage) {
+                L.res_partial = nullptr;
+                L.dt_partial = nullptr;
             }
         }
         __syncthreads();
-        if (!s_go) continue;
-        const StageLaunch& L = *reinterpret_cast<const StageLaunch*>(s_rec + s_sel * W);
-        if (L.mode < 0) continue;
-        stage_body<FLUX, ORDER, NS, FT>(L, tm.y);
     }
-    if (threadIdx.x == 0 && atomicAdd(&ctr[1], 1) == (int)gridDim.x - 1) {
-        atomicExch(&ctr[0], 0);
-        atomicExch(&ctr[1], 0);
-    }
+    return true;
 }
 
-
-// grid of a persistent launch: as many CTAs as the device holds at once
-// (SMs x resident CTAs per SM), at most one per tile; the occupancy is
-// looked up once per kernel, shared-memory size and device
-template <typename K>
-inline int persistent_grid(K kern, int threads, int smem, int n_tiles) {
-    struct Key {
-        const void* k;
-        int smem, dev;
-        bool operator<(const Key& o) const {
-            return k != o.k ? k < o.k : smem != o.smem ? smem < o.smem : dev < o.dev;
-        }
-    };
-    static std::mutex mu;
-    static std::map<Key, int> cache;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const Key key{reinterpret_cast<const void*>(kern), smem, dev};
-    int slots;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        auto it = cache.find(key);
-        if (it == cache.end()) {
-            int sms = 1, per = 1;
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, threads, smem) != cudaSuccess || per < 1)
-                per = 1;
-            it = cache.emplace(key, sms * per).first;
-        }
-        slots = it->second;
-    }
-    return n_tiles < slots ? n_tiles : slots;
+template <int NS, typename FT>
+__global__ void __maxnreg__(StageShape<FT>::grad_regs)
+    k_grad_batch(const StageLaunch* __restrict__ recs, const int4* __restrict__ tmap, int rk_mode, int stage) {
+    __shared__ __align__(16) unsigned char rec[sizeof(StageLaunch)];
+    StageLaunch& L = *reinterpret_cast<StageLaunch*>(rec);
+    const int4 e = tmap[blockIdx.x];
+    if (!batch_record(recs, e, rk_mode, stage, L)) return;
+    if (L.limiter == 1) grad_body<1, NS, FT>(L, e.y);
+    else grad_body<2, NS, FT>(L, e.y);
 }
 
+template <int FLUX, int ORDER, int NS, typename FT>
+__global__ void __maxnreg__(NS ? StageShape<FT>::regs_ns : StageShape<FT>::regs)
+    k_flux_batch(const StageLaunch* __restrict__ recs, const int4* __restrict__ tmap, int rk_mode, int stage) {
+    __shared__ __align__(16) unsigned char rec[sizeof(StageLaunch)];
+    StageLaunch& L = *reinterpret_cast<StageLaunch*>(rec);
+    const int4 e = tmap[gridDim.x - 1 - blockIdx.x];
+    if (!batch_record(recs, e, rk_mode, stage, L)) return;
+    flux_body<FLUX, ORDER, NS, FT>(L, e.y);
+}
+
+// dynamic shared memory of a k_flux CTA: the tile's face fluxes, overlaid by
+// the last stage's reduction
 template <typename FT>
-inline int stage_smem_bytes_t(const TileDev& T) {
-    using V4 = typename Vec<FT>::v4;
-    using V2 = typename Vec<FT>::v2;
-    return (int)(sizeof(V4) * (T.max_e + 2 * T.max_g) + sizeof(V2) * (T.max_hs + (T.max_hs & 1)) +
-                 sizeof(V4) * T.max_f);
+inline int stage_smem_bytes_t(int max_f, int threads) {
+    const int flux = (int)sizeof(typename Vec<FT>::v4) * max_f, red = (int)sizeof(double) * 6 * threads;
+    return flux > red ? flux : red;
 }
+
+// gradient kernels (gradients.cu, gradients_mixed.cu)
+void launch_grad_fp64(const StageLaunch& L, cudaStream_t st);
+void launch_grad_fp32(const StageLaunch& L, cudaStream_t st);
+void launch_grad_batch_fp64(const BatchLaunch& B, cudaStream_t st);
+void launch_grad_batch_fp32(const BatchLaunch& B, cudaStream_t st);
 
 // per-flux entry points (stage_fNN.cu)
 #define CCFD_DECLARE_FLUX(ID)                                             \

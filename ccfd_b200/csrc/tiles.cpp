@@ -4,9 +4,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <functional>
-#include <memory>
-#include <mutex>
 #include <stdint.h>
 #include <thread>
 
@@ -113,259 +110,104 @@ void ccfd_rcm_order(const ccfd_mesh* m, std::vector<int>& cell_order) {
     cell_order.assign(order.rbegin(), order.rend());
 }
 
-namespace {
-
-// tiles [ta, tb) built by one thread: their concatenated arrays and per-tile
-// sizes; u_code entries go straight into the shared array (disjoint ranges)
-struct TilePart {
-    std::vector<int> counts, e_ref, f_id, f_lr, f_hs, n_e, n_hs, n_f;
-    std::vector<int16_t> hs_nbl, hs_loc;
-    int max_e = 0, max_g = 0, max_hs = 0, max_f = 0;
-};
-
-// per-thread work arrays, reused across calls (a pool shared by all calls):
-// fresh cell- and face-sized arrays per thread and call cost more in page
-// faults than the tile construction
-struct TileScratch {
-    std::vector<int> loc, gloc, fmark, E, R1, R2, G, faces, bfaces;
-    TilePart part;
-};
-std::mutex g_scratch_mu;
-std::vector<std::unique_ptr<TileScratch>> g_scratch;
-
-std::unique_ptr<TileScratch> take_scratch() {
-    std::lock_guard<std::mutex> lk(g_scratch_mu);
-    if (g_scratch.empty()) return std::unique_ptr<TileScratch>(new TileScratch());
-    std::unique_ptr<TileScratch> s = std::move(g_scratch.back());
-    g_scratch.pop_back();
-    return s;
+// Host work split into ranges of tiles, one thread each; every range writes
+// to its own entries, so the result does not depend on the thread count.
+template <typename Fn>
+static void tile_ranges(int n_tiles, Fn fn) {
+    const unsigned hw = std::thread::hardware_concurrency();
+    const int nth = std::max(1, std::min((int)std::min(hw ? hw : 1u, 16u), n_tiles / 64));
+    std::vector<std::thread> pool;
+    for (int k = 0; k + 1 < nth; ++k)
+        pool.emplace_back(fn, (int)((long)n_tiles * k / nth), (int)((long)n_tiles * (k + 1) / nth));
+    fn((int)((long)n_tiles * (nth - 1) / nth), n_tiles);
+    for (std::thread& th : pool) th.join();
 }
 
-void give_scratch(std::unique_ptr<TileScratch> s) {
-    std::lock_guard<std::mutex> lk(g_scratch_mu);
-    g_scratch.push_back(std::move(s));
-}
-
-void build_range(const ccfd_mesh* m, const std::vector<int>& cperm, const std::vector<int>& cinv,
-                 const std::vector<int>& fdev, int T, int ta, int tb, const std::vector<long>& dh,
-                 std::vector<int>& u_code, TileScratch& W) {
-    const long N = m->n_cells, F = m->n_faces, B = m->n_bc;
-    std::vector<int>&loc = W.loc, &gloc = W.gloc, &fmark = W.fmark;
-    std::vector<int>&E = W.E, &R1 = W.R1, &R2 = W.R2, &G = W.G, &faces = W.faces, &bfaces = W.bfaces;
-    loc.assign(N, -1);
-    gloc.assign(B, -1);
-    fmark.assign(F, -1);
-    TilePart& P = W.part;
-    P.counts.clear();
-    P.e_ref.clear();
-    P.f_id.clear();
-    P.f_lr.clear();
-    P.f_hs.clear();
-    P.n_e.clear();
-    P.n_hs.clear();
-    P.n_f.clear();
-    P.hs_nbl.clear();
-    P.hs_loc.clear();
-    P.max_e = P.max_g = P.max_hs = P.max_f = 0;
-    for (int t = ta; t < tb; ++t) {
-        long d0 = (long)t * T, d1 = std::min(N, d0 + T);
-        E.clear();
-        R1.clear();
-        R2.clear();
-        G.clear();
-        faces.clear();
-        bfaces.clear();
-        for (long d = d0; d < d1; ++d) {
-            loc[d] = (int)E.size();
-            E.push_back((int)d);
-        }
-        auto add_nbrs = [&](long d, std::vector<int>& out) {
-            long c = cperm[d];
-            for (long h = m->hs_offset[c]; h < m->hs_offset[c + 1]; ++h) {
-                long nb = m->hs_nb[h];
-                if (nb < 0) continue;
-                int nd = cinv[nb];
-                if (loc[nd] < 0) {
-                    loc[nd] = -2;  // claimed
-                    out.push_back(nd);
-                }
-            }
-        };
-        for (long d = d0; d < d1; ++d) add_nbrs(d, R1);
-        for (int d : R1) {
-            loc[d] = (int)E.size();
-            E.push_back(d);
-        }
-        for (int d : R1) add_nbrs(d, R2);
-        for (int d : R2) {
-            loc[d] = (int)E.size();
-            E.push_back(d);
-        }
-        const int nT = (int)(d1 - d0), nG = nT + (int)R1.size(), nEc = (int)E.size();
-        // ghosts adjacent to gradient cells
-        for (int i = 0; i < nG; ++i) {
-            long c = cperm[E[i]];
-            for (long h = m->hs_offset[c]; h < m->hs_offset[c + 1]; ++h) {
-                long nb = m->hs_nb[h];
-                if (nb >= 0) continue;
-                int g = (int)(-1 - nb);
-                if (gloc[g] < 0) {
-                    gloc[g] = (int)(E.size() + G.size());
-                    G.push_back(g);
-                }
-            }
-        }
-        // gradient half-sides: local neighbour index per half-side
-        const size_t hs_nbl0 = P.hs_nbl.size();
-        const int blk = (int)P.hs_loc.size();
-        int hs_local = 0;
-        for (int i = 0; i < nG; ++i) {
-            P.hs_loc.push_back((int16_t)hs_local);
-            long c = cperm[E[i]];
-            for (long h = m->hs_offset[c]; h < m->hs_offset[c + 1]; ++h, ++hs_local) {
-                long nb = m->hs_nb[h];
-                int l = nb >= 0 ? loc[cinv[nb]] : gloc[-1 - nb];
-                P.hs_nbl.push_back((int16_t)l);
-            }
-        }
-        P.hs_loc.push_back((int16_t)hs_local);
-        // faces touching tile cells in first-encounter order: interior
-        // faces first, then the tile's boundary faces
-        for (long d = d0; d < d1; ++d) {
-            long c = cperm[d];
-            for (long h = m->hs_offset[c]; h < m->hs_offset[c + 1]; ++h) {
-                long f = m->hs_face[h];
-                if (m->hs_nb[h] < 0) {
-                    bfaces.push_back((int)f);
-                    continue;
-                }
-                if (fmark[f] != t) {
-                    fmark[f] = t;
-                    faces.push_back((int)f);
-                }
-            }
-        }
-        const int nFi = (int)faces.size();
-        faces.insert(faces.end(), bfaces.begin(), bfaces.end());
-        for (size_t j = 0; j < faces.size(); ++j) {
-            long f = faces[j];
-            long o = m->face_cells[2 * f], nbr = m->face_cells[2 * f + 1];
-            int il = loc[cinv[o]];
-            int hl = P.hs_loc[blk + il] + (int)(m->face_hs[2 * f] - m->hs_offset[o]);
-            if ((int)j < nFi) {
-                int ir = loc[cinv[nbr]];
-                int hr = P.hs_loc[blk + ir] + (int)(m->face_hs[2 * f + 1] - m->hs_offset[nbr]);
-                P.f_id.push_back(fdev[f]);
-                P.f_lr.push_back(il | (ir << 16));
-                P.f_hs.push_back(hl | (hr << 16));
-            } else {
-                int g = (int)(-1 - nbr);
-                P.f_id.push_back(-1 - g);
-                P.f_lr.push_back(il | (gloc[g] << 16));
-                P.f_hs.push_back(hl);
-            }
-            fmark[f] = -3 - (int)j;  // local index for the codes below
-        }
-        for (long d = d0; d < d1; ++d) {
-            long c = cperm[d];
-            long k = dh[d];
-            for (long h = m->hs_offset[c]; h < m->hs_offset[c + 1]; ++h, ++k) {
-                int j = -3 - fmark[m->hs_face[h]];
-                u_code[k] = 2 * j + (m->hs_sign[h] > 0 ? 0 : 1);
-            }
-        }
-        for (size_t j = 0; j < faces.size(); ++j) fmark[faces[j]] = t;
-        P.counts.push_back(nT);
-        P.counts.push_back(nG);
-        P.counts.push_back(nEc);
-        P.counts.push_back((int)(E.size() + G.size()));
-        for (int d : E) P.e_ref.push_back(d);
-        for (int g : G) P.e_ref.push_back(-1 - g);
-        P.n_e.push_back((int)(E.size() + G.size()));
-        P.n_hs.push_back((int)(P.hs_nbl.size() - hs_nbl0));
-        P.n_f.push_back((int)faces.size());
-        P.max_e = std::max(P.max_e, (int)(E.size() + G.size()));
-        P.max_g = std::max(P.max_g, nG);
-        P.max_hs = std::max(P.max_hs, hs_local);
-        P.max_f = std::max(P.max_f, (int)faces.size());
-        // reset the local maps
-        for (int d : E) loc[d] = -1;
-        for (int g : G) gloc[g] = -1;
-    }
-}
-
-template <typename V>
-void append(V& dst, const V& src) {
-    dst.insert(dst.end(), src.begin(), src.end());
-}
-
-}  // namespace
-
-// Tiles are independent: ranges of tiles are built on several host threads
-// (each with its own scratch) and concatenated in tile order, so the result
-// does not depend on the thread count.
-void ccfd_build_tiles(const ccfd_mesh* m, const std::vector<int>& cperm, const std::vector<int>& cinv,
-                      const std::vector<int>& fdev, int T, TileSet& ts) {
-    const long N = m->n_cells;
+void ccfd_build_tiles(const ccfd_mesh* m, const std::vector<int>& cperm, const std::vector<int>& cinv, int T,
+                      TileSet& ts) {
+    const long N = m->n_cells, F = m->n_faces;
     // (the vectors keep their capacity from an earlier call)
-    ts.e_off.clear();
-    ts.counts.clear();
-    ts.e_ref.clear();
-    ts.hs_off.clear();
-    ts.hs_nbl.clear();
-    ts.hs_loc.clear();
-    ts.f_off.clear();
-    ts.f_id.clear();
-    ts.f_lr.clear();
-    ts.f_hs.clear();
-    ts.max_e = ts.max_g = ts.max_hs = ts.max_f = 0;
     ts.tile_cells = T;
     ts.n_tiles = (int)((N + T - 1) / T);
-    // device half-side offsets (device cell order keeps each cell's
-    // reference side order)
-    std::vector<long> dh(N + 1);
-    dh[0] = 0;
-    for (long d = 0; d < N; ++d) {
-        long c = cperm[d];
-        dh[d + 1] = dh[d] + (m->hs_offset[c + 1] - m->hs_offset[c]);
-    }
-    ts.u_code.assign(dh[N], 0);
-    unsigned hw = std::thread::hardware_concurrency();
-    int nth = (int)std::max(1u, std::min(hw ? hw : 1u, 16u));
-    nth = std::max(1, std::min(nth, ts.n_tiles / 64));
-    std::vector<std::unique_ptr<TileScratch>> work(nth);
-    for (int k = 0; k < nth; ++k) work[k] = take_scratch();
-    std::vector<std::thread> pool;
-    for (int k = 0; k < nth; ++k) {
-        int ta = (int)((long)ts.n_tiles * k / nth), tb = (int)((long)ts.n_tiles * (k + 1) / nth);
-        if (k + 1 == nth)
-            build_range(m, cperm, cinv, fdev, T, ta, tb, dh, ts.u_code, *work[k]);
-        else
-            pool.emplace_back(build_range, m, std::cref(cperm), std::cref(cinv), std::cref(fdev), T, ta, tb,
-                              std::cref(dh), std::ref(ts.u_code), std::ref(*work[k]));
-    }
-    for (std::thread& th : pool) th.join();
-    ts.e_off.push_back(0);
-    ts.hs_off.push_back(0);
-    ts.f_off.push_back(0);
-    for (int k = 0; k < nth; ++k) {
-        const TilePart& P = work[k]->part;
-        append(ts.counts, P.counts);
-        append(ts.e_ref, P.e_ref);
-        append(ts.hs_nbl, P.hs_nbl);
-        append(ts.hs_loc, P.hs_loc);
-        append(ts.f_id, P.f_id);
-        append(ts.f_lr, P.f_lr);
-        append(ts.f_hs, P.f_hs);
-        for (size_t i = 0; i < P.n_e.size(); ++i) {
-            ts.e_off.push_back(ts.e_off.back() + P.n_e[i]);
-            ts.hs_off.push_back(ts.hs_off.back() + P.n_hs[i]);
-            ts.f_off.push_back(ts.f_off.back() + P.n_f[i]);
+    ts.own_off.assign(ts.n_tiles + 1, 0);
+    ts.border_off.assign(ts.n_tiles + 1, 0);
+    ts.face_of.resize(F);
+    ts.id_of.resize(F);
+    ts.u_code.resize(4 * (size_t)N);
+    // A side's face is new to the tile when this is the face's first side in
+    // device order within the tile: the other side's cell is in another tile
+    // or later (or the same cell's later side, on a periodic mesh); it is the
+    // tile's own when the other side's cell is not in an earlier tile.
+    auto classify = [&](long d, long h, long d0, long* f) {
+        *f = m->hs_face[h];
+        const long nb = m->hs_nb[h];
+        if (nb < 0) return 1;
+        const long e = cinv[nb];
+        if (e < d0) return 2;                          // border: owned by an earlier tile
+        if (e >= d0 + T || e > d) return 1;            // own, first seen here
+        if (e == d) {                                  // a cell that is its own neighbour: the first of its sides
+            const long s0 = m->face_hs[2 * *f], s1 = m->face_hs[2 * *f + 1];
+            return h == std::min(s0, s1) ? 1 : 0;
         }
-        ts.max_e = std::max(ts.max_e, P.max_e);
-        ts.max_g = std::max(ts.max_g, P.max_g);
-        ts.max_hs = std::max(ts.max_hs, P.max_hs);
-        ts.max_f = std::max(ts.max_f, P.max_f);
+        return 0;                                      // already seen in this tile
+    };
+    tile_ranges(ts.n_tiles, [&](int ta, int tb) {
+        for (int t = ta; t < tb; ++t) {
+            const long d0 = (long)t * T, d1 = std::min(N, d0 + T);
+            int own = 0, border = 0;
+            for (long d = d0; d < d1; ++d)
+                for (long h = m->hs_offset[cperm[d]]; h < m->hs_offset[cperm[d] + 1]; ++h) {
+                    long f;
+                    const int c = classify(d, h, d0, &f);
+                    own += c == 1;
+                    border += c == 2;
+                }
+            ts.own_off[t + 1] = own;
+            ts.border_off[t + 1] = border;
+        }
+    });
+    ts.max_f = 0;
+    for (int t = 0; t < ts.n_tiles; ++t) {
+        ts.max_f = std::max(ts.max_f, ts.own_off[t + 1] + ts.border_off[t + 1]);
+        ts.own_off[t + 1] += ts.own_off[t];
+        ts.border_off[t + 1] += ts.border_off[t];
     }
-    for (int k = 0; k < nth; ++k) give_scratch(std::move(work[k]));
+    ts.border.resize(ts.border_off[ts.n_tiles]);
+    tile_ranges(ts.n_tiles, [&](int ta, int tb) {
+        for (int t = ta; t < tb; ++t) {
+            const long d0 = (long)t * T, d1 = std::min(N, d0 + T);
+            int id = ts.own_off[t];
+            for (long d = d0; d < d1; ++d)
+                for (long h = m->hs_offset[cperm[d]]; h < m->hs_offset[cperm[d] + 1]; ++h) {
+                    long f;
+                    if (classify(d, h, d0, &f) == 1) {
+                        ts.face_of[id] = (int)f;
+                        ts.id_of[f] = id++;
+                    }
+                }
+        }
+    });
+    tile_ranges(ts.n_tiles, [&](int ta, int tb) {
+        for (int t = ta; t < tb; ++t) {
+            const long d0 = (long)t * T, d1 = std::min(N, d0 + T);
+            const int own0 = ts.own_off[t], n_own = ts.own_off[t + 1] - own0;
+            int nb = ts.border_off[t];
+            for (long d = d0; d < d1; ++d) {
+                uint16_t* code = &ts.u_code[4 * (size_t)d];
+                int k = 0;
+                for (long h = m->hs_offset[cperm[d]]; h < m->hs_offset[cperm[d] + 1]; ++h, ++k) {
+                    long f;
+                    int local;
+                    if (classify(d, h, d0, &f) == 2) {
+                        local = n_own + (nb - ts.border_off[t]);
+                        ts.border[nb++] = ts.id_of[f];
+                    } else {
+                        local = ts.id_of[f] - own0;
+                    }
+                    code[k] = (uint16_t)(2 * local + (m->hs_sign[h] > 0 ? 0 : 1));
+                }
+                for (; k < 4; ++k) code[k] = 0xffff;
+            }
+        }
+    });
 }
