@@ -76,6 +76,8 @@ enum Ctl {
     CTL_WORDS = 8
 };
 
+struct SweepRec;
+
 // Device descriptor of one member (pointers into its context and state).
 struct ImpDev {
     long N;
@@ -90,7 +92,7 @@ struct ImpDev {
     float4 *Vf, *Zf, *dxsf;
     float *Dinvf, *Of;
     double4* rjb;  // mixed precision: R(U, t) of the FP32-flux evaluation, base of the Jacobian columns
-    int* flag;  // [0] GMRES cycle done, [1] final m, [2] singular, [3] non-finite
+    int* flag;  // [0] GMRES cycle done, [1] final m, [2] singular, [3] non-finite, [4] a sweep gave up
     int* ctl;   // Ctl words
     Ctrl* ctrl;
     const int *hs_off, *hs_nb, *twin;
@@ -102,6 +104,10 @@ struct ImpDev {
     // their off-diagonal blocks in side order, -1 padded to four
     const int *lev_f_off, *fw_cell, *lev_b_off, *bw_cell;
     const int4 *fw_nb, *fw_h, *bw_nb, *bw_h;
+    // forward / backward sequences of the cluster kernel's warps: chunk
+    // offsets [kClWorkers + 1], records (8 per chunk)
+    const int* cl_off[2];
+    const SweepRec* cl_rec[2];
 };
 
 struct ImpState {
@@ -129,6 +135,9 @@ struct ImpState {
     int n_lev_f = 0, n_lev_b = 0, max_level = 0;
     int *lev_f_off = nullptr, *fw_cell = nullptr, *lev_b_off = nullptr, *bw_cell = nullptr;
     int4 *fw_nb = nullptr, *fw_h = nullptr, *bw_nb = nullptr, *bw_h = nullptr;
+    bool cluster_ok = false;     // the sweeps fit the cluster kernel
+    int* cl_off[2] = {nullptr, nullptr};
+    SweepRec* cl_rec[2] = {nullptr, nullptr};
     bool ready = false;
     void* solo = nullptr;        // the member set of this context running alone
     std::vector<int> hs_off_h;   // device CSR offsets of the half-sides (host copy)
@@ -341,7 +350,7 @@ __global__ void kb_gmres_flags(const ImpDev* __restrict__ I) {
     if (threadIdx.x) return;
     int on = newton_on(d);
     d.flag[0] = on ? 0 : 1;
-    d.flag[1] = d.flag[2] = d.flag[3] = 0;
+    d.flag[1] = d.flag[2] = d.flag[3] = d.flag[4] = 0;
     d.ctl[CTL_SKIP_GMRES] = !on;
 }
 
@@ -481,7 +490,7 @@ __global__ void kb_gmres_end(const ImpDev* __restrict__ I) {
     MEMBER;
     if (threadIdx.x || !newton_on(d)) return;
     d.ctl[CTL_GMRES_TOTAL] += min(d.flag[1], d.K - 1) + 1;
-    if (d.flag[3]) fail_member(d, CCFD_ERR_GMRES, FLAG_GMRES);
+    if (d.flag[3] || d.flag[4]) fail_member(d, CCFD_ERR_GMRES, FLAG_GMRES);
 }
 
 // delX += alp[nn] Z[nn], nn = 0..m in order (src/linearSolver.c:482-490);
@@ -822,6 +831,329 @@ __global__ void __launch_bounds__(THREADS) kb_lusgs(const ImpDev* __restrict__ I
     sweep<false, T>(d.n_lev_b, d.lev_b_off, d.bw_cell, d.bw_nb, d.bw_h, B, dx, dx, dxs, Dinv, O);
 }
 
+// ---- LU-SGS on a cluster
+// One member's sweeps by the warps of a cluster, as a pipeline.  On one SM a
+// level costs ~1.5 us: its blocks come through one SM's L2 port, its warps
+// share four schedulers, and every level ends in a barrier.  Here each of
+// kClWorkers pairs of warps owns a contiguous range of the reference's cell
+// numbers and walks its own cells level by level, a chunk of up to eight cells
+// (four threads each) at a time.  A cell needs only cells of lower number
+// (forward) or higher number (backward), so values flow one way between the
+// ranges and the pairs run behind one another without any barrier.  A value
+// of the same pair comes from a ring of its recent results; every other value
+// is stored by its producer into a mailbox in the consumer's shared memory,
+// where the value itself says that it has arrived (mailboxes start as a NaN
+// pattern that no result is stored with).  One warp of a pair brings the
+// blocks in by cp.async, the other computes: with both in one warp a chunk
+// took ~250 instructions of one instruction stream, 1.8 us per level of the
+// 32,768-cell airfoil.  The arithmetic and its order are those of sweep_row;
+// a missing neighbour is a zero block times a zero vector, which changes no
+// sum that starts at +0.  One application on the 32,768-cell airfoil (383 levels
+// each way): 0.45 ms against 1.18 ms by one CTA.
+constexpr int kClCtas = 8, kClPairs = 4, kClWorkers = kClCtas * kClPairs, kClThreads = 64 * kClPairs;
+constexpr int kClRing = 64;         // recent results of a pair (a power of two)
+constexpr int kClMail = 2304;       // mailboxes of a CTA, the first one a zero vector
+constexpr int kClNb = 3;            // most neighbours of a cell on one side of the sweep
+constexpr int kClSlots = 6;         // chunks whose blocks are in shared memory
+constexpr int kClAhead = 3;         // copies in flight, chunks
+constexpr int kClIdx = 16;          // chunks whose records are in shared memory
+static_assert(kClIdx >= kClSlots + 2 * kClAhead + 1, "a record outlives its blocks");
+constexpr int kClSpin = 1 << 20;    // polls before the sweep gives up
+
+// One place of a chunk: cell (-1: none), half-sides of its blocks in side
+// order (-1: none), where the neighbours' values are and where its own result
+// goes besides the ring (byte offsets in the CTA's shared memory, the target
+// with its CTA in the upper bits, -1: none); neighbours and mailboxes of the
+// chunk's busiest place.
+struct alignas(16) SweepRec {
+    int cell, h[kClNb], src[kClNb], n_nb, mail[4], n_mail, pad[3];  // 64 bytes, copied by four threads
+};
+constexpr int kClMailBits = 20;
+constexpr long kClSpareRecs = 16384;  // records of a sweep: at most four per cell and these
+
+// shared memory of a pair and of a CTA, bytes
+template <typename T>
+constexpr int cluster_pair_smem() {
+    return (int)(kClRing * 4 * sizeof(T) + kClIdx * 8 * sizeof(SweepRec) + kClSlots * 8 * 4 * sizeof(T) +
+                 kClSlots * (1 + kClNb) * 32 * 4 * sizeof(T) + 16);
+}
+template <typename T>
+constexpr int cluster_smem() {
+    return (int)(kClMail * 4 * sizeof(T)) + kClPairs * cluster_pair_smem<T>();
+}
+
+__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void cp16(unsigned dst, const void* src, bool take) {
+    // without `take` nothing is read and zeros are written
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(take ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ int ld_acquire(unsigned addr) {
+    int v;
+    asm volatile("ld.acquire.cta.shared::cta.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release(unsigned addr, int v) {
+    asm volatile("st.release.cta.shared::cta.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ unsigned map_rank(unsigned addr, int rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+
+// Values in the ring and the mailboxes: a value whose (upper) word is all ones
+// has not arrived; a result of that pattern is stored as the ordinary NaN.
+__device__ __forceinline__ double arrivable(double v) {
+    return __double2hiint(v) == -1 ? __longlong_as_double(0x7ff8000000000000ll) : v;
+}
+__device__ __forceinline__ float arrivable(float v) {
+    return __float_as_int(v) == -1 ? __int_as_float(0x7fc00000) : v;
+}
+__device__ __forceinline__ void put_value(unsigned addr, double v) {
+    asm volatile("st.relaxed.cluster.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+}
+__device__ __forceinline__ void put_value(unsigned addr, float v) {
+    asm volatile("st.relaxed.cluster.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+// the four components at addr; false if one has not arrived
+__device__ __forceinline__ bool get_values(unsigned addr, double x[4]) {
+    asm volatile("ld.relaxed.cluster.shared::cta.v2.f64 {%0, %1}, [%2];" : "=d"(x[0]), "=d"(x[1]) : "r"(addr) : "memory");
+    asm volatile("ld.relaxed.cluster.shared::cta.v2.f64 {%0, %1}, [%2];"
+                 : "=d"(x[2]), "=d"(x[3])
+                 : "r"(addr + 16)
+                 : "memory");
+    const unsigned a = max((unsigned)__double2hiint(x[0]), (unsigned)__double2hiint(x[1]));
+    const unsigned b = max((unsigned)__double2hiint(x[2]), (unsigned)__double2hiint(x[3]));
+    return max(a, b) != ~0u;
+}
+__device__ __forceinline__ bool get_values(unsigned addr, float x[4]) {
+    asm volatile("ld.relaxed.cluster.shared::cta.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3])
+                 : "r"(addr)
+                 : "memory");
+    const unsigned a = max(__float_as_uint(x[0]), __float_as_uint(x[1]));
+    const unsigned b = max(__float_as_uint(x[2]), __float_as_uint(x[3]));
+    return max(a, b) != ~0u;
+}
+
+// wait until the other warp's counter at addr is at least `want`; `seen` keeps
+// the last value read.  False after kClSpin polls (the whole warp alike).
+__device__ __forceinline__ bool reach(unsigned addr, int want, int& seen) {
+    for (int n = 0; seen < want; ++n) {
+        if (n == kClSpin) return false;
+        seen = __shfl_sync(0xffffffffu, ld_acquire(addr), 0);
+    }
+    return true;
+}
+
+// layout of a pair's shared memory from its base
+template <typename T>
+struct PairSmem {
+    unsigned ring, idx, own, rows, full, done;
+    __device__ explicit PairSmem(unsigned base) {
+        ring = base;                                                    // [kClRing][4]
+        idx = ring + (unsigned)(kClRing * 4 * sizeof(T));               // [kClIdx][8] records
+        own = idx + (unsigned)(kClIdx * 8 * sizeof(SweepRec));          // [kClSlots][8][4]
+        rows = own + (unsigned)(kClSlots * 8 * 4 * sizeof(T));          // [kClSlots][1 + kClNb][units][32] of 16 bytes
+        full = rows + (unsigned)(kClSlots * (1 + kClNb) * 32 * 4 * sizeof(T));  // chunks copied
+        done = full + 4;                                                // chunks computed
+    }
+};
+template <typename T>
+constexpr int kRowUnits = (int)(4 * sizeof(T) / 16);  // 16-byte units of a block row
+template <typename T>
+constexpr unsigned kSlotBytes = (unsigned)((1 + kClNb) * 32 * 4 * sizeof(T));
+
+// the copying warp of a pair
+template <typename T>
+__device__ __forceinline__ bool cluster_copy(const PairSmem<T>& S, const int nck, const SweepRec* __restrict__ rec,
+                                             const T* own_src, const T* __restrict__ Dinv, const T* __restrict__ O) {
+    constexpr int U = kRowUnits<T>;
+    const int lane = threadIdx.x & 31, quad = lane >> 2, a = lane & 3;
+    auto fetch_idx = [&](int c) {
+        if (c < nck)
+            cp16(S.idx + (unsigned)((c % kClIdx) * 8 * sizeof(SweepRec)) + 16 * lane,
+                 reinterpret_cast<const char*>(rec + 8 * (long)c) + 16 * lane, true);
+    };
+    for (int c = 0; c < 2 * kClAhead; ++c) fetch_idx(c);
+    cp_commit();
+    cp_wait<0>();
+    __syncwarp();
+    int done = 0, slot = 0;
+    for (int c = 0; c < nck + kClAhead - 1; ++c) {
+        if (c < nck) {
+            // the slot's last chunk has been computed
+            if (!reach(S.done, c - kClSlots + 1, done)) return false;
+            const unsigned r = S.idx + (unsigned)(((c % kClIdx) * 8 + quad) * sizeof(SweepRec));
+            int cell, h[kClNb];
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(cell), "=r"(h[0]), "=r"(h[1]), "=r"(h[2])
+                         : "r"(r)
+                         : "memory");
+            const bool have = cell >= 0;
+            const long cl = have ? cell : 0;
+            const unsigned row = S.rows + slot * kSlotBytes<T> + 16 * lane;
+            const char* d = reinterpret_cast<const char*>(Dinv + 16 * cl + 4 * a);
+#pragma unroll
+            for (int u = 0; u < U; ++u) cp16(row + 512 * u, d + 16 * u, have);
+#pragma unroll
+            for (int q = 0; q < kClNb; ++q) {
+                const char* o = reinterpret_cast<const char*>(O + 16 * (long)max(h[q], 0) + 4 * a);
+#pragma unroll
+                for (int u = 0; u < U; ++u) cp16(row + 512 * ((q + 1) * U + u), o + 16 * u, h[q] >= 0);
+            }
+            if (a < U)
+                cp16(S.own + (unsigned)((slot * 8 + quad) * 4 * sizeof(T)) + 16 * a,
+                     reinterpret_cast<const char*>(own_src + 4 * cl) + 16 * a, have);
+            fetch_idx(c + 2 * kClAhead);
+            slot = slot + 1 == kClSlots ? 0 : slot + 1;
+        }
+        cp_commit();
+        if (c >= kClAhead - 1) {
+            cp_wait<kClAhead - 1>();
+            __syncwarp();
+            if (lane == 0) st_release(S.full, c - kClAhead + 2);
+        }
+    }
+    return true;
+}
+
+// the computing warp of a pair
+template <bool FWD, typename T>
+__device__ __forceinline__ bool cluster_compute(const PairSmem<T>& S, const unsigned cta, const int nck, T* dst) {
+    constexpr int U = kRowUnits<T>;
+    const int lane = threadIdx.x & 31, quad = lane >> 2, a = lane & 3, lane0 = lane & ~3;
+    int full = 0, slot = 0;
+    for (int c = 0; c < nck; ++c) {
+        if (!reach(S.full, c + 1, full)) return false;
+        __syncwarp();  // also orders the last chunk's results in the ring
+        const unsigned rp = S.idx + (unsigned)(((c % kClIdx) * 8 + quad) * sizeof(SweepRec));
+        int cell, src[kClNb], n_nb, mail[4], n_mail, skip[3];
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(cell), "=r"(skip[0]), "=r"(skip[1]), "=r"(skip[2])
+                     : "r"(rp)
+                     : "memory");
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(src[0]), "=r"(src[1]), "=r"(src[2]), "=r"(n_nb)
+                     : "r"(rp + 16)
+                     : "memory");
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(mail[0]), "=r"(mail[1]), "=r"(mail[2]), "=r"(mail[3])
+                     : "r"(rp + 32)
+                     : "memory");
+        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(n_mail) : "r"(rp + 48) : "memory");
+        const unsigned row = S.rows + slot * kSlotBytes<T> + 16 * lane;
+        auto get_row = [&](int q, T v[4]) {
+            if constexpr (sizeof(T) == 8) {
+                asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "r"(row + 512 * q * U) : "memory");
+                asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];"
+                             : "=d"(v[2]), "=d"(v[3])
+                             : "r"(row + 512 * (q * U + 1))
+                             : "memory");
+            } else {
+                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                             : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                             : "r"(row + 512 * q)
+                             : "memory");
+            }
+        };
+        T o[kClNb][4], di[4], own_a;
+#pragma unroll
+        for (int q = 0; q < kClNb; ++q) get_row(q + 1, o[q]);
+        get_row(0, di);
+        const unsigned oa = S.own + (unsigned)(((slot * 8 + quad) * 4 + a) * sizeof(T));
+        if constexpr (sizeof(T) == 8) asm volatile("ld.shared.f64 %0, [%1];" : "=d"(own_a) : "r"(oa) : "memory");
+        else asm volatile("ld.shared.f32 %0, [%1];" : "=f"(own_a) : "r"(oa) : "memory");
+        T t1a = T(0.0);
+#pragma unroll
+        for (int q = 0; q < kClNb; ++q)
+            if (q < n_nb) {  // the same for the whole warp
+                T x[4];
+                const unsigned at = cta + (unsigned)src[q];
+                for (int n = 0; !__all_sync(0xffffffffu, get_values(at, x)); ++n)
+                    if (n == kClSpin) return false;
+#pragma unroll
+                for (int b = 0; b < 4; ++b) t1a += o[q][b] * x[b];
+            }
+        __syncwarp();
+        const T w = FWD ? own_a - t1a : t1a;
+        T t2 = T(0.0);
+#pragma unroll
+        for (int b = 0; b < 4; ++b) t2 += di[b] * __shfl_sync(0xffffffffu, w, lane0 + b);
+        const T res = FWD ? t2 : own_a - t2;
+        const T out = arrivable(res);
+        put_value(S.ring + (unsigned)((4 * ((8 * c + quad) & (kClRing - 1)) + a) * sizeof(T)), out);
+        for (int j = 0; j < n_mail; ++j) {  // the same for the whole warp
+            const int to = j == 0 ? mail[0] : j == 1 ? mail[1] : j == 2 ? mail[2] : mail[3];
+            if (to >= 0)
+                put_value(map_rank(cta + (unsigned)(to & ((1 << kClMailBits) - 1)) + (unsigned)(a * sizeof(T)),
+                                   to >> kClMailBits),
+                          out);
+        }
+        if (cell >= 0) __stcg(dst + 4 * (long)cell + a, res);
+        slot = slot + 1 == kClSlots ? 0 : slot + 1;
+        __syncwarp();
+        if (lane == 0) st_release(S.done, c + 1);
+    }
+    return true;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kClThreads) kb_lusgs_cluster(const ImpDev* __restrict__ I, int m) {
+    extern __shared__ __align__(16) unsigned char cl_smem[];
+    const ImpDev& d = I[blockIdx.x / kClCtas];
+    if (!d.precond || !gmres_on(d) || d.fp32 != (sizeof(T) == 4)) return;  // the whole cluster alike
+    const int warp = threadIdx.x >> 5, pair = warp >> 1, w = (blockIdx.x % kClCtas) * kClPairs + pair;
+    const unsigned cta = smem_u32(cl_smem);
+    const PairSmem<T> S(cta + (unsigned)(kClMail * 4 * sizeof(T)) + pair * cluster_pair_smem<T>());
+    const T *B, *Dinv, *O;
+    T *dxs, *dx;
+    if constexpr (sizeof(T) == 8) {
+        B = reinterpret_cast<const T*>(d.V + (long)m * d.N);
+        dxs = reinterpret_cast<T*>(d.dxs);
+        dx = reinterpret_cast<T*>(d.Z + (long)m * d.N);
+        Dinv = reinterpret_cast<const T*>(d.Dinv);
+        O = reinterpret_cast<const T*>(d.O);
+    } else {
+        B = reinterpret_cast<const T*>(d.Vf + (long)m * d.N);
+        dxs = reinterpret_cast<T*>(d.dxsf);
+        dx = reinterpret_cast<T*>(d.Zf + (long)m * d.N);
+        Dinv = reinterpret_cast<const T*>(d.Dinvf);
+        O = reinterpret_cast<const T*>(d.Of);
+    }
+    bool ok = true;
+    for (int s = 0; s < 2; ++s) {  // forward, backward
+        constexpr int kWords = (int)(kClMail * 4 * sizeof(T) / 16), kZero = kRowUnits<T>;
+        for (int k = threadIdx.x; k < kWords; k += kClThreads)
+            reinterpret_cast<int4*>(cl_smem)[k] = k < kZero ? make_int4(0, 0, 0, 0) : make_int4(-1, -1, -1, -1);
+        if ((threadIdx.x & 63) == 0) {
+            st_release(S.full, 0);
+            st_release(S.done, 0);
+        }
+        // every CTA has started, with empty mailboxes; the forward result is
+        // complete before the backward sweep requests it
+        cluster_sync();
+        const int c0 = d.cl_off[s][w], nck = d.cl_off[s][w + 1] - c0;
+        const SweepRec* rec = d.cl_rec[s] + 8 * (long)c0;
+        bool mine;
+        if (warp & 1) mine = cluster_copy<T>(S, nck, rec, s ? dxs : B, Dinv, O);
+        else if (s == 0) mine = cluster_compute<true, T>(S, cta, nck, dxs);
+        else mine = cluster_compute<false, T>(S, cta, nck, dx);
+        ok = ok && mine;
+        cp_wait<0>();
+        cluster_sync();  // no store into a CTA's memory is still to come
+    }
+    if (!ok) d.flag[4] = 1;
+}
+
 // number of members whose Newton loop (what = 0) / GMRES cycle (what = 1)
 // is still running
 __global__ void kb_count(const ImpDev* __restrict__ I, int n, int what, int* out) {
@@ -1006,6 +1338,91 @@ int ccfd_implicit_setup(ccfd_ctx* ctx, const std::vector<int>& hs_off, const std
         std::vector<int4> fwn, fwh, bwn, bwh;
         pack(lfc, lo_off, lo_nb, lo_h, fwn, fwh);
         pack(lbc, up_off, up_nb, up_h, bwn, bwh);
+        // the cluster kernel's sequences; a numbering that needs more
+        // mailboxes than a CTA has stays with the single-CTA kernel
+        S->cluster_ok = true;
+        auto sequences = [&](const std::vector<int>& lev, const std::vector<int>& cells, const std::vector<int4>& pn,
+                             const std::vector<int4>& ph, std::vector<int>& off, std::vector<SweepRec>& recs) {
+            // cells arrive level by level; each goes to the warp that owns
+            // its reference number, into the warp's last chunk if that is of
+            // the same level and has room
+            std::vector<int> place(N), n_ck(kClWorkers, 0), fill(kClWorkers, 8), last(kClWorkers, -1);
+            auto owner = [&](int d) { return (int)((long)ref[d] * kClWorkers / N); };
+            for (long k = 0; k < N; ++k) {
+                const int d = cells[k], w = owner(d);
+                if (fill[w] == 8 || last[w] != lev[d]) {
+                    ++n_ck[w];
+                    fill[w] = 0;
+                    last[w] = lev[d];
+                }
+                place[d] = 8 * (n_ck[w] - 1) + fill[w]++;
+            }
+            off.assign(kClWorkers + 1, 0);
+            for (int w = 0; w < kClWorkers; ++w) off[w + 1] = off[w] + n_ck[w];
+            // (a numbering whose chunks stay nearly empty is left out too:
+            // its records would outgrow the memory estimate)
+            if (8L * off[kClWorkers] > 4 * N + kClSpareRecs) S->cluster_ok = false;
+            if (!S->cluster_ok) return;
+            // byte offsets in a CTA's shared memory
+            const int word = S->fp32 ? 16 : 32;  // a result
+            const int pair_bytes = S->fp32 ? cluster_pair_smem<float>() : cluster_pair_smem<double>();
+            SweepRec none;
+            memset(&none, 0, sizeof(none));
+            none.cell = -1;
+            for (int q = 0; q < kClNb; ++q) none.h[q] = -1;  // src 0: the zero vector
+            for (int q = 0; q < 4; ++q) none.mail[q] = -1;
+            recs.assign(8 * (size_t)off[kClWorkers], none);
+            std::vector<int> used(kClCtas, 1);
+            for (long k = 0; k < N; ++k) {
+                const int d = cells[k], w = owner(d), cta = w / kClPairs;
+                SweepRec& r = recs[8 * (size_t)off[w] + place[d]];
+                r.cell = d;
+                const int *n4 = &pn[k].x, *h4 = &ph[k].x;
+                for (int q = 0; q < 4; ++q) {
+                    if (n4[q] < 0) continue;
+                    if (q >= kClNb) {
+                        S->cluster_ok = false;
+                        continue;
+                    }
+                    r.h[q] = h4[q];
+                    const int e = n4[q], we = owner(e);
+                    // the ring holds the last kClRing places before the end
+                    // of this chunk
+                    if (we == w && place[e] >= (place[d] | 7) + 1 - kClRing) {
+                        r.src[q] = word * kClMail + (w % kClPairs) * pair_bytes + word * (place[e] & (kClRing - 1));
+                    } else if (used[cta] < kClMail) {
+                        const int box = word * used[cta]++;
+                        r.src[q] = box;
+                        SweepRec& from = recs[8 * (size_t)off[we] + place[e]];
+                        int j = 0;
+                        while (j < 3 && from.mail[j] >= 0) ++j;  // a cell has at most four neighbours
+                        from.mail[j] = (cta << kClMailBits) | box;
+                    } else {
+                        S->cluster_ok = false;
+                    }
+                }
+            }
+            for (size_t c = 0; c < recs.size() / 8; ++c) {
+                int nn = 0, nm = 0;
+                for (int k = 0; k < 8; ++k) {
+                    const SweepRec& r = recs[8 * c + k];
+                    for (int q = 0; q < kClNb; ++q)
+                        if (r.h[q] >= 0) nn = std::max(nn, q + 1);
+                    for (int q = 0; q < 4; ++q)
+                        if (r.mail[q] >= 0) nm = std::max(nm, q + 1);
+                }
+                for (int k = 0; k < 8; ++k) {
+                    recs[8 * c + k].n_nb = nn;
+                    recs[8 * c + k].n_mail = nm;
+                }
+            }
+        };
+        std::vector<int> clo[2];
+        std::vector<SweepRec> clr[2];
+        sequences(lf, lfc, fwn, fwh, clo[0], clr[0]);
+        sequences(lb, lbc, bwn, bwh, clo[1], clr[1]);
+        for (int k = 0; k < 2 && S->cluster_ok; ++k)
+            if ((st = iupload(ctx, &S->cl_off[k], clo[k])) || (st = iupload(ctx, &S->cl_rec[k], clr[k]))) return st;
         S->n_lev_f = nlf;
         S->n_lev_b = nlb;
         for (int l = 0; l < nlf; ++l) S->max_level = std::max(S->max_level, lfo[l + 1] - lfo[l]);
@@ -1047,6 +1464,7 @@ struct ImpSet {
     int n = 0, max_nb = 0, max_col = 0, max_colsize = 0, max_K = 0, max_newton = 0;
     int max_level = 0;  // widest LU-SGS level (cells) over the members
     bool any_precond = false;
+    bool cluster = false;  // LU-SGS by clusters
     bool pc64 = false, pc32 = false;  // preconditioned members in FP64 / FP32
     int* d_count = nullptr;
     int* h_count = nullptr;
@@ -1112,6 +1530,10 @@ static ImpDev make_dev(ccfd_ctx* ctx) {
     d.color_cells = S->color_cells;
     d.n_lev_f = S->n_lev_f; d.n_lev_b = S->n_lev_b;
     d.lev_f_off = S->lev_f_off; d.fw_cell = S->fw_cell; d.fw_nb = S->fw_nb; d.fw_h = S->fw_h;
+    for (int k = 0; k < 2; ++k) {
+        d.cl_off[k] = S->cl_off[k];
+        d.cl_rec[k] = S->cl_rec[k];
+    }
     d.lev_b_off = S->lev_b_off; d.bw_cell = S->bw_cell; d.bw_nb = S->bw_nb; d.bw_h = S->bw_h;
     return d;
 }
@@ -1122,6 +1544,14 @@ static int set_build(const std::vector<ccfd_ctx*>& members, cudaStream_t stream,
     M->members = members;
     M->n = (int)members.size();
     M->stream = stream;
+    M->cluster = true;
+    for (ccfd_ctx* ctx : members) M->cluster = M->cluster && ((ImpState*)ctx->implicit_state)->cluster_ok;
+    if (M->cluster) {
+        CKM(cudaFuncSetAttribute(kb_lusgs_cluster<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 cluster_smem<double>()));
+        CKM(cudaFuncSetAttribute(kb_lusgs_cluster<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 cluster_smem<float>()));
+    }
     std::vector<ImpDev> hd;
     std::map<std::tuple<int, int, int, int, int>, std::vector<int>> by_variant;
     for (int k = 0; k < M->n; ++k) {
@@ -1267,6 +1697,33 @@ static void build_jacobian(ImpSet* M, cudaStream_t st) {
     kb_jac_finish<<<gv, kB, 0, st>>>(M->dev);
 }
 
+// LU-SGS of Krylov vector m of every member, a cluster each.  Two implicit
+// steps of the first n airfoils of the batched set took, with clusters / one
+// CTA per member (ms): n = 16 84 / 180, 32 114 / 196, 64 190 / 273, 128 384 /
+// 526; one CTA per member is left to numberings that need more mailboxes than
+// a CTA has.
+template <typename T>
+static int launch_lusgs(ImpSet* M, int m, cudaStream_t st) {
+    if (!M->cluster) {
+        kb_lusgs<kSweepThreads, T><<<M->n, kSweepThreads, 0, st>>>(M->dev, m);
+        return CCFD_OK;
+    }
+    constexpr int smem = cluster_smem<T>();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(M->n * kClCtas);
+    cfg.blockDim = dim3(kClThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = kClCtas;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    CKM(cudaLaunchKernelEx(&cfg, kb_lusgs_cluster<T>, (const ImpDev*)M->dev, m));
+    return CCFD_OK;
+}
+
 static int count_on(ImpSet* M, int what, int* out) {
     kb_count<<<1, 256, 0, M->stream>>>(M->dev, M->n, what, M->d_count);
     CKM(cudaMemcpyAsync(M->h_count, M->d_count, sizeof(int), cudaMemcpyDeviceToHost, M->stream));
@@ -1299,8 +1756,8 @@ static int set_step(ImpSet* M) {
             kb_jac_check<<<g1, 32, 0, st>>>(M->dev);
         }
         for (int m = 0; m < M->max_K; ++m) {
-            if (M->pc64) kb_lusgs<kSweepThreads, double><<<M->n, kSweepThreads, 0, st>>>(M->dev, m);
-            if (M->pc32) kb_lusgs<kSweepThreads, float><<<M->n, kSweepThreads, 0, st>>>(M->dev, m);
+            if (M->pc64 && (s = launch_lusgs<double>(M, m, st))) return s;
+            if (M->pc32 && (s = launch_lusgs<float>(M, m, st))) return s;
             kb_copy_vz<<<gv, kB, 0, st>>>(M->dev, m);
             // matrixVector: epsFD = sqrt(eps) / |Z|
             kb_dot_zz<<<gv, kB, 0, st>>>(M->dev, m);
@@ -1530,20 +1987,25 @@ extern "C" int ccfd_lusgs(ccfd_ctx* ctx, const double* b, double* x) {
     } else {
         CK(cudaMemcpyAsync(S->V, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, st));
     }
+    CK(cudaMemsetAsync(S->flag + 4, 0, sizeof(int), st));
     int ctl[CTL_WORDS] = {0};  // GMRES "on": the sweep runs
     CK(cudaMemcpyAsync(S->ctl, ctl, sizeof(ctl), cudaMemcpyHostToDevice, st));
     if (S->fp32) {
-        kb_lusgs<kSweepThreads, float><<<M->n, kSweepThreads, 0, st>>>(M->dev, 0);
+        if ((s = launch_lusgs<float>(M, 0, st))) return s;
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(hf.data(), S->Zf, sizeof(float) * hf.size(), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         for (size_t k = 0; k < hf.size(); ++k) h[k] = hf[k];
     } else {
-        kb_lusgs<kSweepThreads, double><<<M->n, kSweepThreads, 0, st>>>(M->dev, 0);
+        if ((s = launch_lusgs<double>(M, 0, st))) return s;
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(h.data(), S->Z, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
     }
+    int gave_up = 0;
+    CK(cudaMemcpyAsync(&gave_up, S->flag + 4, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (gave_up) return CCFD_ERR_GMRES;
     for (long d = 0; d < N; ++d) memcpy(x + 4 * (size_t)ctx->cell_of_dev[d], &h[4 * d], sizeof(double) * 4);
     return CCFD_OK;
 }

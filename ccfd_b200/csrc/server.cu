@@ -81,8 +81,10 @@ extern "C" int ccfd_estimate_device_bytes(const ccfd_params* p, const ccfd_mesh*
     if (p->implicit) {
         const double K = (double)(p->n_kdim > 0 ? p->n_kdim : 1);
         // Krylov bases V (K+1) and Z (K), eight work vectors, D / D^-1 per
-        // cell, off-diagonal blocks per half-side, colouring and sweep lists
-        b += (64.0 * K + 32.0 + 8.0 * 32.0 + 256.0 + 96.0) * N + 144.0 * H;
+        // cell, off-diagonal blocks per half-side, colouring and sweep lists,
+        // the cluster sweeps' records (two sweeps of at most 4 N + 16384
+        // records of 64 bytes)
+        b += (64.0 * K + 32.0 + 8.0 * 32.0 + 256.0 + 96.0) * N + 144.0 * H + 128.0 * (4.0 * N + 16384.0);
     }
     *bytes = round_up((size_t)(1.2 * b));
     return CCFD_OK;
