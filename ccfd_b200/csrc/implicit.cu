@@ -83,7 +83,8 @@ struct ImpDev {
     long N;
     int K, nb, precond, n_newton;
     double gam1, eps_gmres, eps2newton;
-    double4 *XK, *Q, *RXK, *F, *dX, *W, *V, *Z, *ptmp, *ut, *dxs, *cons, *prim, *pert;
+    double4 *XK, *Q, *RXK, *F, *dX, *W, *V, *Z, *ptmp, *ut, *dxs, *cons, *prim;
+    double4 *pert[4], *utj[4];  // Jacobian columns: perturbed states and their residuals, one per variable
     double *D, *Dinv, *O, *sc, *partial;
     // mixed precision (fp32 = 1): Krylov basis V, Z, the sweep vector and the
     // LU-SGS blocks D^-1, O in FP32 (Vf, Zf, dxsf, Dinvf, Of instead of the
@@ -121,6 +122,10 @@ struct ImpState {
     float4 *Vf = nullptr, *Zf = nullptr, *dxsf = nullptr;
     float *Dinvf = nullptr, *Of = nullptr;
     double4* RJB = nullptr;      // mixed precision: base residual of the Jacobian columns
+    // the four columns of a colour, evaluated by the same launches: state,
+    // residual, reconstruction and ghost scratch of each
+    double4 *jpert[4] = {}, *jut[4] = {}, *jghost[4] = {};
+    void* jrec[4] = {};
     double* sc = nullptr;        // device scalars
     int* flag = nullptr;         // [0] gmres done, [1] m_final, [2] singular, [3] non-finite
     int* ctl = nullptr;          // Ctl words
@@ -555,64 +560,75 @@ __device__ __forceinline__ double jac_eps(const ImpDev& d) {
     return d.fp32 ? sqrt((double)FLT_EPSILON) : sqrt(DBL_EPSILON);
 }
 
-// gate of colour c: members that build a preconditioner and have colour c
-__global__ void kb_jac_gate(const ImpDev* __restrict__ I, int c) {
-    MEMBER;
-    if (threadIdx.x) return;
-    d.ctl[CTL_SKIP_JAC] = !(newton_on(d) && d.precond && c < d.ncol);
+// member builds a preconditioner and has colour c
+__device__ __forceinline__ bool jac_on(const ImpDev& d, int c) {
+    return newton_on(d) && d.precond && c >= 0 && c < d.ncol;
 }
 
-// perturbed copy of the state (buildMatrix works on a copy of pVar)
+// perturbed copies of the state, one per variable (buildMatrix works on a
+// copy of pVar)
 __global__ void kb_jac_copy(const ImpDev* __restrict__ I) {
     MEMBER;
     if (!newton_on(d) || !d.precond) return;
     CELL_INDEX;
-    if (i < d.N) d.pert[i] = d.prim[i];
+    if (i >= d.N) return;
+    const double4 q = d.prim[i];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) d.pert[v][i] = q;
 }
 
-// perturb (add) or restore variable v of the cells of colour c
-__global__ void kb_jac_perturb(const ImpDev* __restrict__ I, int c, int v, int add) {
+// Between the evaluations of colours c - 1 and c: record the columns of the
+// cells of colour c - 1 (the diagonal block of each and the off-diagonal
+// blocks of its face neighbours, src/linearSolver.c:203-222), restore their
+// states, perturb the cells of colour c and set the skip word of its
+// evaluation.  Five threads per cell, the cell itself and its sides; a thread
+// has all four columns of its block, so it writes whole block rows.
+constexpr int kJacParts = 5;
+
+__global__ void __launch_bounds__(128) kb_jac_next(const ImpDev* __restrict__ I, int c) {
     MEMBER;
-    if (d.ctl[CTL_SKIP_JAC]) return;
-    const int off = d.color_off[c], n = d.color_off[c + 1] - off;
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
+    const int k = (int)(blockIdx.x * blockDim.x + threadIdx.x) / kJacParts;
+    const int part = (int)(blockIdx.x * blockDim.x + threadIdx.x) % kJacParts;
+    const bool next = jac_on(d, c);
+    if (blockIdx.x == 0 && threadIdx.x == 0) d.ctl[CTL_SKIP_JAC] = !next;
     const double reps = jac_eps(d);
-    int cell = d.color_cells[off + k];
-    double q[4];
-    ld(d.prim[cell], q);
-    if (add) q[v] += reps;
-    d.pert[cell] = mk(q);
-}
-
-// record column v of the diagonal block of each perturbed cell and of the
-// off-diagonal blocks of its face neighbours (src/linearSolver.c:203-222)
-__global__ void kb_jac_collect(const ImpDev* __restrict__ I, int c, int v) {
-    MEMBER;
-    if (d.ctl[CTL_SKIP_JAC]) return;
-    const int off = d.color_off[c], n = d.color_off[c + 1] - off;
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const double sreps = 1.0 / jac_eps(d);
-    const double4* base = d.fp32 ? d.rjb : d.RXK;
-    int cell = d.color_cells[off + k];
-    double u[4], r[4];
-    ld(d.ut[cell], u);
-    ld(base[cell], r);
+    if (next && part < 4 && k < d.color_off[c + 1] - d.color_off[c]) {
+        const int cell = d.color_cells[d.color_off[c] + k];
+        double q[4];
+        ld(d.prim[cell], q);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) d.D[16 * (long)cell + 4 * j + v] = 0.0 + (u[j] - r[j]) * sreps;
-    for (int h = d.hs_off[cell]; h < d.hs_off[cell + 1]; ++h) {
-        int e = d.hs_nb[h];
-        if (e < 0) continue;
-        ld(d.ut[e], u);
-        ld(base[e], r);
-        long t = d.twin[h];
+        for (int v = 0; v < 4; ++v)
+            if (v == part) q[v] += reps;
+        d.pert[part][cell] = mk(q);
+    }
+    if (!jac_on(d, c - 1) || k >= d.color_off[c] - d.color_off[c - 1]) return;
+    const int cell = d.color_cells[d.color_off[c - 1] + k];
+    if (part < 4) d.pert[part][cell] = d.prim[cell];
+    // the block this thread records: rows of cell e, columns of `cell`
+    int e = cell;
+    long t = 16 * (long)cell;
+    if (part > 0) {
+        const int h = d.hs_off[cell] + part - 1;
+        if (h >= d.hs_off[cell + 1]) return;
+        e = d.hs_nb[h];
+        if (e < 0) return;
+        t = 16 * (long)d.twin[h];
+    }
+    const double sreps = 1.0 / reps;
+    double r[4], u[4][4];
+    ld(d.fp32 ? d.rjb[e] : d.RXK[e], r);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const double o = 0.0 + (u[j] - r[j]) * sreps;
-            if (d.fp32) d.Of[16 * t + 4 * j + v] = (float)o;
-            else d.O[16 * t + 4 * j + v] = o;
-        }
+    for (int v = 0; v < 4; ++v) ld(d.utj[v][e], u[v]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        double o[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) o[v] = 0.0 + (u[v][j] - r[j]) * sreps;
+        if (part == 0) *reinterpret_cast<double4*>(d.D + t + 4 * j) = mk(o);
+        else if (d.fp32)
+            *reinterpret_cast<float4*>(d.Of + t + 4 * j) =
+                make_float4((float)o[0], (float)o[1], (float)o[2], (float)o[3]);
+        else *reinterpret_cast<double4*>(d.O + t + 4 * j) = mk(o);
     }
 }
 
@@ -1249,6 +1265,38 @@ int ccfd_implicit_setup(ccfd_ctx* ctx, const std::vector<int>& hs_off, const std
                    (st = ialloc(ctx, &S->dxs, N))) {
             return st;
         }
+        // Scratch of the four columns of a colour.  The Krylov vectors are idle
+        // while the Jacobian is built (V_1 .. V_K are written by the
+        // iterations after it, Z_0 .. by theirs), so the columns live there
+        // as far as they fit.
+        {
+            const size_t vec = S->fp32 ? sizeof(float4) : sizeof(double4);
+            char* at[2] = {S->fp32 ? (char*)(S->Vf + N) : (char*)(S->V + N), S->fp32 ? (char*)S->Zf : (char*)S->Z};
+            size_t left[2] = {vec * K * (size_t)N, vec * K * (size_t)N};
+            auto take = [&](void** p, size_t bytes) -> int {
+                for (int r = 0; r < 2; ++r) {
+                    const size_t skip = (size_t)(-(intptr_t)at[r]) & 255;
+                    if (skip + bytes <= left[r]) {
+                        *p = at[r] + skip;
+                        at[r] += skip + bytes;
+                        left[r] -= skip + bytes;
+                        return CCFD_OK;
+                    }
+                }
+                char* q = nullptr;
+                const int e = ialloc(ctx, &q, bytes);
+                *p = q;
+                return e;
+            };
+            const bool ns = ctx->params.eqn == CCFD_NAVIER_STOKES;
+            const size_t faces = (size_t)(ctx->mesh.F + ctx->mesh.B);
+            for (int v = 0; v < 4; ++v)
+                if ((st = take((void**)&S->jpert[v], sizeof(double4) * N)) ||
+                    (st = take((void**)&S->jut[v], sizeof(double4) * N)) ||
+                    (ctx->params.spatial_order == 2 && (st = take(&S->jrec[v], 2 * vec * (ns ? (size_t)N : faces)))) ||
+                    (st = ialloc(ctx, &S->jghost[v], 2 * ((size_t)ctx->B + 1))))
+                    return st;
+        }
         // twins
         std::vector<int> twin(H, -1);
         for (long d = 0; d < N; ++d)
@@ -1454,7 +1502,7 @@ struct ImpGroup {
     int n_tiles = 0, smem = 0, smem_jac = 0;
     StageLaunch *rec_mv = nullptr, *rec_nt = nullptr, *rec_jac = nullptr, *rec_jb = nullptr;
     // tile maps of the records: the same tiles with each kind's skip word
-    int4 *tmap_mv = nullptr, *tmap_nt = nullptr, *tmap_jac = nullptr;
+    int4 *tmap_mv = nullptr, *tmap_nt = nullptr, *tmap_jac = nullptr, *tmap_jb = nullptr;
 };
 
 struct ImpSet {
@@ -1483,6 +1531,7 @@ static void set_free(ImpSet* M) {
         cudaFreeAsync(g.tmap_mv, M->stream);
         cudaFreeAsync(g.tmap_nt, M->stream);
         cudaFreeAsync(g.tmap_jac, M->stream);
+        cudaFreeAsync(g.tmap_jb, M->stream);
     }
     if (M->dev) cudaFreeAsync(M->dev, M->stream);
     if (M->d_count) cudaFreeAsync(M->d_count, M->stream);
@@ -1514,7 +1563,10 @@ static ImpDev make_dev(ccfd_ctx* ctx) {
     d.V = S->V; d.Z = S->Z; d.ptmp = S->ptmp; d.ut = S->ut; d.dxs = S->dxs;
     d.cons = ctx->cons0;
     d.prim = ctx->prim_buf[ctx->cur];
-    d.pert = ctx->prim_buf[ctx->cur ^ 1];
+    for (int v = 0; v < 4; ++v) {
+        d.pert[v] = S->jpert[v];
+        d.utj[v] = S->jut[v];
+    }
     d.D = S->D; d.Dinv = S->Dinv; d.O = S->O; d.sc = S->sc; d.partial = S->partial;
     d.fp32 = S->fp32;
     d.Vf = S->Vf; d.Zf = S->Zf; d.dxsf = S->dxsf; d.Dinvf = S->Dinvf; d.Of = S->Of;
@@ -1583,8 +1635,8 @@ static int set_build(const std::vector<ccfd_ctx*>& members, cudaStream_t stream,
         ImpGroup g;
         std::tie(g.flux, g.order, g.ns, g.fp32, g.jac32) = kv.first;
         const std::vector<int>& idx = kv.second;
-        std::vector<StageLaunch> mv(idx.size()), nt(idx.size()), jac(idx.size()), jb(idx.size());
-        std::vector<int4> tm_mv, tm_nt, tm_jac;
+        std::vector<StageLaunch> mv(idx.size()), nt(idx.size()), jac(4 * idx.size()), jb(idx.size());
+        std::vector<int4> tm_mv, tm_nt, tm_jac, tm_jb;
         int max_f = 0;
         for (size_t j = 0; j < idx.size(); ++j) {
             ccfd_ctx* ctx = members[idx[j]];
@@ -1605,20 +1657,29 @@ static int set_build(const std::vector<ccfd_ctx*>& members, cudaStream_t stream,
             L.u_t = S->RXK;
             L.skip = S->ctl + CTL_SKIP_NEWTON;
             nt[j] = L;
-            // Jacobian columns at t
+            // Jacobian columns at t, one record per variable; they leave the
+            // residual partials and the wall pressures of R(XK) alone
             L.a_time = 0.0;
-            L.prim_in = ctx->prim_buf[ctx->cur ^ 1];
-            L.u_t = S->ut;
             L.skip = S->ctl + CTL_SKIP_JAC;
             L.fp32 = g.jac32;
-            jac[j] = L;
+            L.res_partial = nullptr;
+            L.ghost_pface = nullptr;
             // their base in mixed precision: R(U, t) with FP32 fluxes
             L.u_t = S->RJB;
             jb[j] = L;
+            for (int v = 0; v < 4; ++v) {
+                L.prim_in = S->jpert[v];
+                L.u_t = S->jut[v];
+                L.fstate = L.grad = S->jrec[v];
+                L.ghosts.state = S->jghost[v];
+                L.ghosts.face = S->jghost[v] ? S->jghost[v] + ctx->B + 1 : nullptr;
+                jac[4 * j + v] = L;
+            }
             for (int t = 0; t < ctx->tiles.n_tiles; ++t) {
                 tm_mv.push_back(tile_entry((int)j, t, mv[j].skip));
                 tm_nt.push_back(tile_entry((int)j, t, nt[j].skip));
-                tm_jac.push_back(tile_entry((int)j, t, jac[j].skip));
+                for (int v = 0; v < 4; ++v) tm_jac.push_back(tile_entry((int)(4 * j + v), t, jac[4 * j].skip));
+                tm_jb.push_back(tile_entry((int)j, t, jb[j].skip));
             }
             max_f = std::max(max_f, ctx->tiles.max_f);
         }
@@ -1628,7 +1689,7 @@ static int set_build(const std::vector<ccfd_ctx*>& members, cudaStream_t stream,
         size_t rb = sizeof(StageLaunch) * idx.size();
         CKM(ccfd_malloc_async((void**)&g.rec_mv, rb, stream));
         CKM(ccfd_malloc_async((void**)&g.rec_nt, rb, stream));
-        CKM(ccfd_malloc_async((void**)&g.rec_jac, rb, stream));
+        CKM(ccfd_malloc_async((void**)&g.rec_jac, 4 * rb, stream));
         if (g.jac32) {
             CKM(ccfd_malloc_async((void**)&g.rec_jb, rb, stream));
             CKM(cudaMemcpyAsync(g.rec_jb, jb.data(), rb, cudaMemcpyHostToDevice, stream));
@@ -1636,13 +1697,15 @@ static int set_build(const std::vector<ccfd_ctx*>& members, cudaStream_t stream,
         const size_t tb = sizeof(int4) * tm_mv.size();
         CKM(ccfd_malloc_async((void**)&g.tmap_mv, tb, stream));
         CKM(ccfd_malloc_async((void**)&g.tmap_nt, tb, stream));
-        CKM(ccfd_malloc_async((void**)&g.tmap_jac, tb, stream));
+        CKM(ccfd_malloc_async((void**)&g.tmap_jac, 4 * tb, stream));
+        CKM(ccfd_malloc_async((void**)&g.tmap_jb, tb, stream));
+        CKM(cudaMemcpyAsync(g.tmap_jb, tm_jb.data(), tb, cudaMemcpyHostToDevice, stream));
         CKM(cudaMemcpyAsync(g.tmap_mv, tm_mv.data(), tb, cudaMemcpyHostToDevice, stream));
         CKM(cudaMemcpyAsync(g.tmap_nt, tm_nt.data(), tb, cudaMemcpyHostToDevice, stream));
-        CKM(cudaMemcpyAsync(g.tmap_jac, tm_jac.data(), tb, cudaMemcpyHostToDevice, stream));
+        CKM(cudaMemcpyAsync(g.tmap_jac, tm_jac.data(), 4 * tb, cudaMemcpyHostToDevice, stream));
         CKM(cudaMemcpyAsync(g.rec_mv, mv.data(), rb, cudaMemcpyHostToDevice, stream));
         CKM(cudaMemcpyAsync(g.rec_nt, nt.data(), rb, cudaMemcpyHostToDevice, stream));
-        CKM(cudaMemcpyAsync(g.rec_jac, jac.data(), rb, cudaMemcpyHostToDevice, stream));
+        CKM(cudaMemcpyAsync(g.rec_jac, jac.data(), 4 * rb, cudaMemcpyHostToDevice, stream));
         M->groups.push_back(g);
     }
     CKM(cudaStreamSynchronize(stream));
@@ -1660,8 +1723,8 @@ static void residuals(ImpSet* M, RecKind kind) {
         const bool jac = kind == REC_JAC || kind == REC_JB;
         BatchLaunch B;
         B.recs = kind == REC_MV ? g.rec_mv : kind == REC_NT ? g.rec_nt : kind == REC_JAC ? g.rec_jac : g.rec_jb;
-        B.tmap = kind == REC_MV ? g.tmap_mv : kind == REC_NT ? g.tmap_nt : g.tmap_jac;
-        B.n_tiles = g.n_tiles;
+        B.tmap = kind == REC_MV ? g.tmap_mv : kind == REC_NT ? g.tmap_nt : kind == REC_JAC ? g.tmap_jac : g.tmap_jb;
+        B.n_tiles = kind == REC_JAC ? 4 * g.n_tiles : g.n_tiles;
         B.smem_bytes = jac ? g.smem_jac : g.smem;
         B.rk_mode = 0;
         B.stage = 0;
@@ -1674,25 +1737,18 @@ static void residuals(ImpSet* M, RecKind kind) {
 }
 
 // buildMatrix + calcDinv (src/linearSolver.c:186-252, :136-179) of the
-// members that build a preconditioner: a perturbed copy of the state, the
-// base of the mixed-precision columns, every colour and variable, blocks
-// and inverses
+// members that build a preconditioner: perturbed copies of the state, the
+// base of the mixed-precision columns, every colour (its four variables in the
+// same launches), blocks and inverses
 static void build_jacobian(ImpSet* M, cudaStream_t st) {
-    const dim3 gv(M->max_nb, M->n), g1(1, M->n);
+    const dim3 gv(M->max_nb, M->n);
     kb_jac_copy<<<gv, kB, 0, st>>>(M->dev);
-    if (M->pc32) {
-        kb_jac_gate<<<g1, 32, 0, st>>>(M->dev, 0);
-        residuals(M, REC_JB);
-    }
-    const dim3 gc((M->max_colsize + kB - 1) / kB, M->n);
+    const dim3 gc((kJacParts * M->max_colsize + 127) / 128, M->n);
+    kb_jac_next<<<gc, 128, 0, st>>>(M->dev, 0);
+    if (M->pc32) residuals(M, REC_JB);
     for (int c = 0; c < M->max_col; ++c) {
-        kb_jac_gate<<<g1, 32, 0, st>>>(M->dev, c);
-        for (int v = 0; v < 4; ++v) {
-            kb_jac_perturb<<<gc, kB, 0, st>>>(M->dev, c, v, 1);
-            residuals(M, REC_JAC);
-            kb_jac_collect<<<gc, kB, 0, st>>>(M->dev, c, v);
-            kb_jac_perturb<<<gc, kB, 0, st>>>(M->dev, c, v, 0);
-        }
+        residuals(M, REC_JAC);
+        kb_jac_next<<<gc, 128, 0, st>>>(M->dev, c + 1);
     }
     kb_jac_finish<<<gv, kB, 0, st>>>(M->dev);
 }

@@ -85,6 +85,11 @@ extern "C" int ccfd_estimate_device_bytes(const ccfd_params* p, const ccfd_mesh*
         // the cluster sweeps' records (two sweeps of at most 4 N + 16384
         // records of 64 bytes)
         b += (64.0 * K + 32.0 + 8.0 * 32.0 + 256.0 + 96.0) * N + 144.0 * H + 128.0 * (4.0 * N + 16384.0);
+        // the Jacobian's four columns, as far as the Krylov vectors (idle
+        // meanwhile) do not hold them, and their ghosts
+        const double vec = p->precision == CCFD_MIXED ? 16.0 : 32.0;
+        const double cols = 4.0 * (64.0 * N + 2.0 * vec * (p->eqn == CCFD_NAVIER_STOKES ? N : F));
+        b += 256.0 * B + (cols > 1.8 * K * vec * N ? cols : 0.0);
     }
     *bytes = round_up((size_t)(1.2 * b));
     return CCFD_OK;
