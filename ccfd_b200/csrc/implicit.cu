@@ -1088,18 +1088,21 @@ __device__ __forceinline__ bool cluster_compute(const PairSmem<T>& S, const unsi
         const unsigned oa = S.own + (unsigned)(((slot * 8 + quad) * 4 + a) * sizeof(T));
         if constexpr (sizeof(T) == 8) asm volatile("ld.shared.f64 %0, [%1];" : "=d"(own_a) : "r"(oa) : "memory");
         else asm volatile("ld.shared.f32 %0, [%1];" : "=f"(own_a) : "r"(oa) : "memory");
+        T x[kClNb][4];
+        for (int n = 0;; ++n) {
+            bool here = true;
+#pragma unroll
+            for (int q = 0; q < kClNb; ++q)
+                if (q < n_nb) here = get_values(cta + (unsigned)src[q], x[q]) && here;  // n_nb: the warp's
+            if (__all_sync(0xffffffffu, here)) break;
+            if (n == kClSpin) return false;
+        }
         T t1a = T(0.0);
 #pragma unroll
         for (int q = 0; q < kClNb; ++q)
-            if (q < n_nb) {  // the same for the whole warp
-                T x[4];
-                const unsigned at = cta + (unsigned)src[q];
-                for (int n = 0; !__all_sync(0xffffffffu, get_values(at, x)); ++n)
-                    if (n == kClSpin) return false;
+            if (q < n_nb)
 #pragma unroll
-                for (int b = 0; b < 4; ++b) t1a += o[q][b] * x[b];
-            }
-        __syncwarp();
+                for (int b = 0; b < 4; ++b) t1a += o[q][b] * x[q][b];
         const T w = FWD ? own_a - t1a : t1a;
         T t2 = T(0.0);
 #pragma unroll
