@@ -673,6 +673,19 @@ __global__ void k_state_out(int n, const double4* __restrict__ src, const int* _
     if (c < n) dst[c] = src[dev_of_cell[c]];
 }
 
+// gradients in the reference's cell order, (x of the four variables, y of the
+// four) per cell
+__global__ void k_grad_out(int n, const double4* __restrict__ grad, const int* __restrict__ dev_of_cell,
+                           double4* __restrict__ dst) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= n) return;
+    // stored variable by variable (ld_grad in stage_impl.cuh)
+    const size_t d = (size_t)dev_of_cell[c];
+    const double4 a = grad[2 * d], b = grad[2 * d + 1];
+    dst[2 * (size_t)c] = make_double4(a.x, a.z, b.x, b.z);
+    dst[2 * (size_t)c + 1] = make_double4(a.y, a.w, b.y, b.w);
+}
+
 extern "C" int ccfd_set_state(ccfd_ctx* ctx, const double* state, int kind) {
     if (!ctx || !state || !ctx->uploaded) return CCFD_ERR_ARG;
     if (ctx->batch) return CCFD_ERR_BUSY;
@@ -772,26 +785,25 @@ extern "C" int ccfd_residual(ccfd_ctx* ctx, double time, double* u_t_out, double
     CK(cudaSetDevice(ctx->device));
     int st = ccfd_residual_device(ctx, time, grad_out != nullptr);
     if (st) return st;
+    // permuted to the reference's order on the device, then one copy straight
+    // into each caller's array (a host loop over the cells took 0.8 of the
+    // call's 1.5 ms at 63,000 cells)
     const long N = ctx->N;
+    const unsigned nb = (unsigned)((N + 255) / 256);
     if (u_t_out) {
-        std::vector<double4> h(N);
-        CK(cudaMemcpyAsync(h.data(), ctx->u_t, sizeof(double4) * N, cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        for (long d = 0; d < N; ++d) {
-            double* s = &u_t_out[4 * ctx->cell_of_dev[d]];
-            s[0] = h[d].x; s[1] = h[d].y; s[2] = h[d].z; s[3] = h[d].w;
-        }
+        k_state_out<<<nb, 256, 0, ctx->stream>>>((int)N, ctx->u_t, ctx->d_dev_of_cell, ctx->xfer);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(u_t_out, ctx->xfer, sizeof(double4) * N, cudaMemcpyDeviceToHost, ctx->stream));
     }
     if (grad_out) {
-        std::vector<double4> h(2 * N);
-        CK(cudaMemcpyAsync(h.data(), ctx->grad, sizeof(double4) * 2 * N, cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        for (long d = 0; d < N; ++d) {
-            double* s = &grad_out[8 * ctx->cell_of_dev[d]];
-            // stored variable by variable (ld_grad in stage_impl.cuh)
-            s[0] = h[2 * d].x; s[1] = h[2 * d].z; s[2] = h[2 * d + 1].x; s[3] = h[2 * d + 1].z;
-            s[4] = h[2 * d].y; s[5] = h[2 * d].w; s[6] = h[2 * d + 1].y; s[7] = h[2 * d + 1].w;
-        }
+        double4* tmp = nullptr;
+        CK(ccfd_malloc_async((void**)&tmp, sizeof(double4) * 2 * N, ctx->stream));
+        k_grad_out<<<nb, 256, 0, ctx->stream>>>((int)N, ctx->grad, ctx->d_dev_of_cell, tmp);
+        cudaError_t e = cudaGetLastError();
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(grad_out, tmp, sizeof(double4) * 2 * N, cudaMemcpyDeviceToHost, ctx->stream);
+        cudaFreeAsync(tmp, ctx->stream);
+        CK(e);
     }
     return check_flags(ctx);
 }

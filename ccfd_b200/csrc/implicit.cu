@@ -1173,6 +1173,27 @@ __global__ void __launch_bounds__(kClThreads) kb_lusgs_cluster(const ImpDev* __r
     if (!ok) d.flag[4] = 1;
 }
 
+// a vector from / to the reference's cell order (FP32 storage: f)
+__global__ void k_vec_in(int n, const double4* __restrict__ src, const int* __restrict__ cell_of_dev,
+                         double4* __restrict__ v, float4* __restrict__ f) {
+    const int d = blockIdx.x * blockDim.x + threadIdx.x;
+    if (d >= n) return;
+    const double4 x = src[cell_of_dev[d]];
+    if (f) f[d] = make_float4((float)x.x, (float)x.y, (float)x.z, (float)x.w);
+    else v[d] = x;
+}
+__global__ void k_vec_out(int n, const double4* __restrict__ v, const float4* __restrict__ f,
+                          const int* __restrict__ dev_of_cell, double4* __restrict__ dst) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= n) return;
+    if (f) {
+        const float4 x = f[dev_of_cell[c]];
+        dst[c] = make_double4(x.x, x.y, x.z, x.w);
+    } else {
+        dst[c] = v[dev_of_cell[c]];
+    }
+}
+
 // number of members whose Newton loop (what = 0) / GMRES cycle (what = 1)
 // is still running
 __global__ void kb_count(const ImpDev* __restrict__ I, int n, int what, int* out) {
@@ -2037,36 +2058,21 @@ extern "C" int ccfd_lusgs(ccfd_ctx* ctx, const double* b, double* x) {
     if (s) return s;
     cudaStream_t st = ctx->stream;
     const long N = S->N;
-    std::vector<double> h(4 * N);
-    for (long d = 0; d < N; ++d) memcpy(&h[4 * d], b + 4 * (size_t)ctx->cell_of_dev[d], sizeof(double) * 4);
-    std::vector<float> hf;
-    if (S->fp32) {
-        hf.assign(h.begin(), h.end());
-        CK(cudaMemcpyAsync(S->Vf, hf.data(), sizeof(float) * hf.size(), cudaMemcpyHostToDevice, st));
-    } else {
-        CK(cudaMemcpyAsync(S->V, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, st));
-    }
+    // b and x pass through the transfer buffer in the reference's order and
+    // are permuted (and rounded) on the device
+    const unsigned nb = (unsigned)((N + kB - 1) / kB);
+    CK(cudaMemcpyAsync(ctx->xfer, b, sizeof(double4) * N, cudaMemcpyHostToDevice, st));
+    k_vec_in<<<nb, kB, 0, st>>>((int)N, ctx->xfer, ctx->d_cell_of_dev, S->V, S->Vf);
     CK(cudaMemsetAsync(S->flag + 4, 0, sizeof(int), st));
-    int ctl[CTL_WORDS] = {0};  // GMRES "on": the sweep runs
-    CK(cudaMemcpyAsync(S->ctl, ctl, sizeof(ctl), cudaMemcpyHostToDevice, st));
-    if (S->fp32) {
-        if ((s = launch_lusgs<float>(M, 0, st))) return s;
-        CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(hf.data(), S->Zf, sizeof(float) * hf.size(), cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        for (size_t k = 0; k < hf.size(); ++k) h[k] = hf[k];
-    } else {
-        if ((s = launch_lusgs<double>(M, 0, st))) return s;
-        CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(h.data(), S->Z, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-    }
+    CK(cudaMemsetAsync(S->ctl, 0, sizeof(int) * CTL_WORDS, st));  // GMRES "on": the sweep runs
+    if ((s = S->fp32 ? launch_lusgs<float>(M, 0, st) : launch_lusgs<double>(M, 0, st))) return s;
+    k_vec_out<<<nb, kB, 0, st>>>((int)N, S->Z, S->Zf, ctx->d_dev_of_cell, ctx->xfer);
+    CK(cudaGetLastError());
     int gave_up = 0;
+    CK(cudaMemcpyAsync(x, ctx->xfer, sizeof(double4) * N, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(&gave_up, S->flag + 4, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    if (gave_up) return CCFD_ERR_GMRES;
-    for (long d = 0; d < N; ++d) memcpy(x + 4 * (size_t)ctx->cell_of_dev[d], &h[4 * d], sizeof(double) * 4);
-    return CCFD_OK;
+    return gave_up ? CCFD_ERR_GMRES : CCFD_OK;
 }
 
 // ---------------------------------------------------------------- batching
