@@ -71,6 +71,29 @@ struct SmemLimit {
     }
 };
 
+// Launch whose CTAs may be set up while the kernel before it on the stream
+// drains (programmatic dependent launch); they wait in grid_wait(), first
+// thing and on every path, so completion stays in stream order.  Microseconds
+// per stage without / with: 8,000 cells 14.15 / 13.65, 32,761 cells 15.15 /
+// 14.60, 500,000 cells 77.8 / 77.0.  The kernels do not release their
+// dependents early: waiting CTAs then take the slots of running ones (16.6 us
+// at 8,000 cells).
+template <typename... P, typename... A>
+inline void launch_dependent(void (*kern)(P...), int grid, int threads, int smem, cudaStream_t st, const A&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, args...);
+}
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // CTA shapes.  k_grad: 4 / grad_vars threads per cell, at most kGradThreads
 // per CTA.
 // k_flux: at most `threads`, `single` unless the context sets another size.
@@ -907,12 +930,14 @@ __device__ __forceinline__ void flux_body(const StageLaunch& L, const int t) {
 // one instance: one tile per CTA, launch parameters in the parameter space
 template <int LIM, int NS, typename FT>
 __global__ void __maxnreg__(StageShape<FT>::grad_regs) k_grad(const __grid_constant__ StageLaunch L) {
+    grid_wait();
     if (inactive(L.ctrl)) return;
     grad_body<LIM, NS, FT>(L, blockIdx.x);
 }
 
 template <int FLUX, int ORDER, int NS, typename FT>
 __global__ void __maxnreg__(NS ? StageShape<FT>::regs_ns : StageShape<FT>::regs) k_flux(const __grid_constant__ StageLaunch L) {
+    grid_wait();
     if (inactive(L.ctrl)) return;
     // last tile first: what k_grad wrote last is still in L2, and the next
     // k_grad starts with the states written last here
@@ -971,6 +996,7 @@ __global__ void __maxnreg__(StageShape<FT>::grad_regs)
     __shared__ __align__(16) unsigned char rec[sizeof(StageLaunch)];
     StageLaunch& L = *reinterpret_cast<StageLaunch*>(rec);
     const int4 e = tmap[blockIdx.x];
+    grid_wait();
     if (!batch_record(recs, e, rk_mode, stage, L)) return;
     if (L.limiter == 1) grad_body<1, NS, FT>(L, e.y);
     else grad_body<2, NS, FT>(L, e.y);
@@ -982,6 +1008,7 @@ __global__ void __maxnreg__(NS ? StageShape<FT>::regs_ns : StageShape<FT>::regs)
     __shared__ __align__(16) unsigned char rec[sizeof(StageLaunch)];
     StageLaunch& L = *reinterpret_cast<StageLaunch*>(rec);
     const int4 e = tmap[gridDim.x - 1 - blockIdx.x];
+    grid_wait();
     if (!batch_record(recs, e, rk_mode, stage, L)) return;
     flux_body<FLUX, ORDER, NS, FT>(L, e.y);
 }
