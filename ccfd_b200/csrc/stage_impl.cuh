@@ -289,15 +289,9 @@ __device__ __forceinline__ void face_flux(const Gas& P, T nx, T ny, T len, const
                                           const T q0[4], const T q1[4], const T g0x[4],
                                           const T g0y[4], const T g1x[4], const T g1y[4], double4 bbd,
                                           T F[4], unsigned* flags) {
-    FluxIn<T> s;
-    s.rL = L[0]; s.uL = nx * L[1] + ny * L[2]; s.vL = -ny * L[1] + nx * L[2]; s.pL = L[3];
-    s.rR = R[0]; s.uR = nx * R[1] + ny * R[2]; s.vR = -ny * R[1] + nx * R[2]; s.pR = R[3];
-    T fc[4];
-    convective_flux<FLUX, T>(P, s, fc, flags);
-    F[0] = fc[0];
-    F[1] = nx * fc[1] - ny * fc[2];
-    F[2] = ny * fc[1] + nx * fc[2];
-    F[3] = fc[3];
+    // the viscous part first: the gradients and cell states (48 values) are
+    // then not live during the convective flux
+    T fv[4] = {T(0.0), T(0.0), T(0.0), T(0.0)};
     if (NS) {
         T st[4], gx[4], gy[4];
         const T bbz = T(bbd.z);
@@ -314,8 +308,20 @@ __device__ __forceinline__ void face_flux(const Gas& P, T nx, T ny, T len, const
         T fdx[4], fdy[4];
         diffusion_flux<T>(P, st, gx, gy, fdx, fdy);
 #pragma unroll
-        for (int v = 0; v < 4; ++v) F[v] -= (fdx[v] * nx + fdy[v] * ny);
+        for (int v = 0; v < 4; ++v) fv[v] = fdx[v] * nx + fdy[v] * ny;
     }
+    FluxIn<T> s;
+    s.rL = L[0]; s.uL = nx * L[1] + ny * L[2]; s.vL = -ny * L[1] + nx * L[2]; s.pL = L[3];
+    s.rR = R[0]; s.uR = nx * R[1] + ny * R[2]; s.vR = -ny * R[1] + nx * R[2]; s.pR = R[3];
+    T fc[4];
+    convective_flux<FLUX, T>(P, s, fc, flags);
+    F[0] = fc[0];
+    F[1] = nx * fc[1] - ny * fc[2];
+    F[2] = ny * fc[1] + nx * fc[2];
+    F[3] = fc[3];
+    if (NS)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) F[v] -= fv[v];
 #pragma unroll
     for (int v = 0; v < 4; ++v) F[v] *= len;
 }
