@@ -129,7 +129,7 @@ struct ImpState {
     double* sc = nullptr;        // device scalars
     int* flag = nullptr;         // [0] gmres done, [1] m_final, [2] singular, [3] non-finite
     int* ctl = nullptr;          // Ctl words
-    double* partial = nullptr;   // per-block partial sums
+    double* partial = nullptr;   // per-block partial sums, two buffers of nb + 1
     int nb = 0;
     // colouring (device cell lists per colour) and neighbour twins
     std::vector<int> color_off;  // host copy of the colour offsets
@@ -177,6 +177,24 @@ __device__ __forceinline__ void block_partial(double v, double* partial) {
         for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
         if (lane == 0) partial[blockIdx.x] = x;
     }
+}
+
+// Sum of a member's nb block partials, the same in every block that asks for
+// it (kB threads, fixed order): the kernel that needs a dot product finishes
+// it itself instead of waiting for a launch in between.
+__device__ __forceinline__ double block_total(const double* partial, int nb) {
+    __shared__ double sh[kB];
+    double v = 0.0;
+    for (int k = threadIdx.x; k < nb; k += kB) v += partial[k];
+    sh[threadIdx.x] = v;
+    __syncthreads();
+    for (int s = kB / 2; s > 0; s >>= 1) {
+        if ((int)threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
+        __syncthreads();
+    }
+    const double r = sh[0];
+    __syncthreads();
+    return r;
 }
 
 // Krylov basis access in the member's precision (FP64 arithmetic outside)
@@ -276,33 +294,12 @@ __global__ void kb_newton_F(const ImpDev* __restrict__ I, int copy_xk) {
     block_partial(v, d.partial);
 }
 
-enum FinalTarget { FT_NORM_X0 = 0, FT_NORM_XK, FT_EPSFD, FT_H };
-
-// fixed-order final reduction of a member's partials; mode 0: sum,
-// 1: sqrt(sum), 2: sqrt(DBL_EPSILON) / sqrt(sum) (the finite-difference step)
-__global__ void kb_final(const ImpDev* __restrict__ I, int target, int row, int col, int mode,
-                         int gmres_gate) {
+// |F|^2 of the Newton loop: into SC_NORM_X0 (first) or SC_NORM_XK
+__global__ void kb_newton_norm(const ImpDev* __restrict__ I, int first) {
     MEMBER;
-    if (gmres_gate ? !gmres_on(d) : !newton_on(d)) return;
-    __shared__ double sh[kB];
-    double v = 0.0;
-    for (int k = threadIdx.x; k < d.nb; k += blockDim.x) v += d.partial[k];
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        double r = sh[0];
-        if (mode == 1) r = sqrt(r);
-        else if (mode == 2) r = sqrt(DBL_EPSILON) / sqrt(r);
-        double* out = target == FT_NORM_X0 ? d.sc + SC_NORM_X0
-                    : target == FT_NORM_XK ? d.sc + SC_NORM_XK
-                    : target == FT_EPSFD   ? d.sc + SC_EPSFD
-                                           : d.sc + SC_H + row * (d.K + 1) + col;
-        *out = r;
-    }
+    if (!newton_on(d)) return;
+    const double r = block_total(d.partial, d.nb);
+    if (threadIdx.x == 0) d.sc[first ? SC_NORM_X0 : SC_NORM_XK] = r;
 }
 
 // eps2newtonLoc and the first test of the Newton loop
@@ -367,8 +364,11 @@ __global__ void kb_copy_vz(const ImpDev* __restrict__ I, int m) {
     if (i < d.N) putZ(d, (long)m * d.N + i, getV(d, (long)m * d.N + i));
 }
 
-__global__ void kb_dot_zz(const ImpDev* __restrict__ I, int m) {
+// |Z_m|^2 partials; also clears the count of members that iterate on
+// (kb_givens counts them)
+__global__ void kb_dot_zz(const ImpDev* __restrict__ I, int m, int* count) {
     MEMBER;
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *count = 0;
     if (!gmres_on(d)) return;
     CELL_INDEX;
     double v = 0.0;
@@ -379,16 +379,18 @@ __global__ void kb_dot_zz(const ImpDev* __restrict__ I, int m) {
     block_partial(v, d.partial);
 }
 
-// U = XK + eps v, pVar = consPrim(U) (src/linearSolver.c:350-360)
+// eps = sqrt(DBL_EPSILON) / |Z_m|; U = XK + eps v, pVar = consPrim(U)
+// (src/linearSolver.c:343-360)
 __global__ void kb_mv_prep(const ImpDev* __restrict__ I, int m) {
     MEMBER;
     if (!gmres_on(d)) return;
     CELL_INDEX;
+    const double e = sqrt(DBL_EPSILON) / sqrt(block_total(d.partial, d.nb));
+    if (i == 0) d.sc[SC_EPSFD] = e;
     if (i >= d.N) return;
     double x[4], z[4], c[4], p[4];
     ld(d.XK[i], x);
     ld(getZ(d, (long)m * d.N + i), z);
-    double e = d.sc[SC_EPSFD];
 #pragma unroll
     for (int k = 0; k < 4; ++k) c[k] = x[k] + e * z[k];
     cons_prim(d.gam1, c, p);
@@ -418,35 +420,44 @@ __global__ void kb_mv_finish(const ImpDev* __restrict__ I, int m) {
     block_partial(dd, d.partial);
 }
 
-// W -= H[nn][m] V_nn (modified Gram-Schmidt step, src/linearSolver.c:
-// 440-450), then the partial of V_{nn+1} . W (or W . W after the last one)
+// H[nn][m] from the partials of V_nn . W; W -= H[nn][m] V_nn (modified
+// Gram-Schmidt step, src/linearSolver.c:440-450), then the partial of
+// V_{nn+1} . W (or W . W after the last one) into the other partial buffer
+// (a member's later blocks may still read this one)
 __global__ void kb_mgs(const ImpDev* __restrict__ I, int nn, int m) {
     MEMBER;
     if (!gmres_on(d)) return;
     CELL_INDEX;
+    double* const in = d.partial + (nn & 1) * (d.nb + 1);
+    double* const out = d.partial + ((nn + 1) & 1) * (d.nb + 1);
+    const double hh = block_total(in, d.nb);
+    if (i == 0) d.sc[SC_H + nn * (d.K + 1) + m] = hh;
     double dd = 0.0;
     if (i < d.N) {
         double w[4], p[4];
         ld(d.W[i], w);
         ld(getV(d, (long)nn * d.N + i), p);
-        double hh = d.sc[SC_H + nn * (d.K + 1) + m];
 #pragma unroll
         for (int k = 0; k < 4; ++k) w[k] -= hh * p[k];
         double4 wv = mk(w);
         d.W[i] = wv;
         dd = nn < m ? cell_dot(getV(d, (long)(nn + 1) * d.N + i), wv) : cell_dot(wv, wv);
     }
-    block_partial(dd, d.partial);
+    block_partial(dd, out);
 }
 
-// Givens rotations, residual estimate and stop test of iteration m, and the
-// back substitution when the cycle ends (src/linearSolver.c:454-481)
-__global__ void kb_givens(const ImpDev* __restrict__ I, int m) {
+// H[m+1][m] = |W|, Givens rotations, residual estimate and stop test of
+// iteration m, and the back substitution when the cycle ends
+// (src/linearSolver.c:452-481); counts the members that iterate on
+__global__ void kb_givens(const ImpDev* __restrict__ I, int m, int* count) {
     MEMBER;
-    if (threadIdx.x || !gmres_on(d)) return;
+    if (!gmres_on(d)) return;
+    const double ww = block_total(d.partial + ((m + 1) & 1) * (d.nb + 1), d.nb);
+    if (threadIdx.x) return;
     const int K = d.K;
     double* sc = d.sc;
     double* H = sc + SC_H;  // H[r * (K + 1) + c]
+    H[(m + 1) * (K + 1) + m] = sqrt(ww);
     double* gam = H + (K + 1) * (K + 1);
     double* C = gam + (K + 1);
     double* S = C + K;
@@ -473,6 +484,8 @@ __global__ void kb_givens(const ImpDev* __restrict__ I, int m) {
         d.flag[1] = m;
         if (!isfinite(alp[0])) d.flag[3] = 1;
         d.ctl[CTL_SKIP_GMRES] = 1;
+    } else {
+        atomicAdd(count, 1);
     }
 }
 
@@ -1194,17 +1207,13 @@ __global__ void k_vec_out(int n, const double4* __restrict__ v, const float4* __
     }
 }
 
-// number of members whose Newton loop (what = 0) / GMRES cycle (what = 1)
-// is still running
-__global__ void kb_count(const ImpDev* __restrict__ I, int n, int what, int* out) {
+// number of members whose Newton loop is still running
+__global__ void kb_count(const ImpDev* __restrict__ I, int n, int* out) {
     __shared__ int cnt;
     if (threadIdx.x == 0) cnt = 0;
     __syncthreads();
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const ImpDev& d = I[k];
-        int on = what ? gmres_on(d) : newton_on(d);
-        if (on) atomicAdd(&cnt, 1);
-    }
+    for (int k = threadIdx.x; k < n; k += blockDim.x)
+        if (newton_on(I[k])) atomicAdd(&cnt, 1);
     __syncthreads();
     if (threadIdx.x == 0) *out = cnt;
 }
@@ -1276,7 +1285,7 @@ int ccfd_implicit_setup(ccfd_ctx* ctx, const std::vector<int>& hs_off, const std
         (st = ialloc(ctx, &S->ptmp, N)) || (st = ialloc(ctx, &S->ut, N)) ||
         (st = ialloc(ctx, &S->sc, SC_H + (K + 1) * (K + 1) + 4 * (K + 1) + 8)) ||
         (st = ialloc(ctx, &S->flag, 8)) || (st = ialloc(ctx, &S->ctl, CTL_WORDS)) ||
-        (st = ialloc(ctx, &S->partial, S->nb + 1)))
+        (st = ialloc(ctx, &S->partial, 2 * ((size_t)S->nb + 1))))
         return st;
     if (ctx->params.precond) {
         if ((st = ialloc(ctx, &S->D, 16 * (size_t)N))) return st;
@@ -1536,6 +1545,7 @@ struct ImpSet {
     int n = 0, max_nb = 0, max_col = 0, max_colsize = 0, max_K = 0, max_newton = 0;
     int max_level = 0;  // widest LU-SGS level (cells) over the members
     bool any_precond = false;
+    bool any_plain = false;  // a member without preconditioner
     bool cluster = false;  // LU-SGS by clusters
     bool pc64 = false, pc32 = false;  // preconditioned members in FP64 / FP32
     int* d_count = nullptr;
@@ -1637,6 +1647,7 @@ static int set_build(const std::vector<ccfd_ctx*>& members, cudaStream_t stream,
         M->max_nb = std::max(M->max_nb, S->nb);
         M->max_K = std::max(M->max_K, S->K);
         M->max_newton = std::max(M->max_newton, ctx->params.n_newton_iter);
+        if (!ctx->params.precond) M->any_plain = true;
         if (ctx->params.precond) {
             M->any_precond = true;
             if (S->fp32) M->pc32 = true;
@@ -1804,8 +1815,10 @@ static int launch_lusgs(ImpSet* M, int m, cudaStream_t st) {
     return CCFD_OK;
 }
 
-static int count_on(ImpSet* M, int what, int* out) {
-    kb_count<<<1, 256, 0, M->stream>>>(M->dev, M->n, what, M->d_count);
+// members whose Newton loop runs (counted here) / whose GMRES cycle runs
+// (counted by the iteration's kb_givens)
+static int count_on(ImpSet* M, bool newton, int* out) {
+    if (newton) kb_count<<<1, 256, 0, M->stream>>>(M->dev, M->n, M->d_count);
     CKM(cudaMemcpyAsync(M->h_count, M->d_count, sizeof(int), cudaMemcpyDeviceToHost, M->stream));
     CKM(cudaStreamSynchronize(M->stream));
     *out = *M->h_count;
@@ -1821,12 +1834,12 @@ static int set_step(ImpSet* M) {
     kb_step_begin<<<gv, kB, 0, st>>>(M->dev);
     residuals(M, REC_NT);
     kb_newton_F<<<gv, kB, 0, st>>>(M->dev, 1);
-    kb_final<<<g1, kB, 0, st>>>(M->dev, FT_NORM_X0, 0, 0, 0, 0);
+    kb_newton_norm<<<g1, kB, 0, st>>>(M->dev, 1);
     kb_newton_start<<<g1, 32, 0, st>>>(M->dev);
     CKM(cudaGetLastError());
     for (int it = 0; it < M->max_newton; ++it) {
         int on = 0, s;
-        if ((s = count_on(M, 0, &on))) return s;
+        if ((s = count_on(M, true, &on))) return s;
         if (!on) break;
         // GMRES_M (src/linearSolver.c:385-510)
         kb_gmres_init<<<gv, kB, 0, st>>>(M->dev);
@@ -1838,30 +1851,25 @@ static int set_step(ImpSet* M) {
         for (int m = 0; m < M->max_K; ++m) {
             if (M->pc64 && (s = launch_lusgs<double>(M, m, st))) return s;
             if (M->pc32 && (s = launch_lusgs<float>(M, m, st))) return s;
-            kb_copy_vz<<<gv, kB, 0, st>>>(M->dev, m);
+            if (M->any_plain) kb_copy_vz<<<gv, kB, 0, st>>>(M->dev, m);
             // matrixVector: epsFD = sqrt(eps) / |Z|
-            kb_dot_zz<<<gv, kB, 0, st>>>(M->dev, m);
-            kb_final<<<g1, kB, 0, st>>>(M->dev, FT_EPSFD, 0, 0, 2, 1);
+            kb_dot_zz<<<gv, kB, 0, st>>>(M->dev, m, M->d_count);
             kb_mv_prep<<<gv, kB, 0, st>>>(M->dev, m);
             residuals(M, REC_MV);
             kb_mv_finish<<<gv, kB, 0, st>>>(M->dev, m);
             // modified Gram-Schmidt
-            for (int nn = 0; nn <= m; ++nn) {
-                kb_final<<<g1, kB, 0, st>>>(M->dev, FT_H, nn, m, 0, 1);
-                kb_mgs<<<gv, kB, 0, st>>>(M->dev, nn, m);
-            }
-            kb_final<<<g1, kB, 0, st>>>(M->dev, FT_H, m + 1, m, 1, 1);
-            kb_givens<<<g1, 32, 0, st>>>(M->dev, m);
+            for (int nn = 0; nn <= m; ++nn) kb_mgs<<<gv, kB, 0, st>>>(M->dev, nn, m);
+            kb_givens<<<g1, kB, 0, st>>>(M->dev, m, M->d_count);
             kb_vnext<<<gv, kB, 0, st>>>(M->dev, m);
             CKM(cudaGetLastError());
-            if ((s = count_on(M, 1, &on))) return s;
+            if ((s = count_on(M, false, &on))) return s;
             if (!on) break;
         }
         kb_gmres_end<<<g1, 32, 0, st>>>(M->dev);
         kb_newton_update<<<gv, kB, 0, st>>>(M->dev);
         residuals(M, REC_NT);
         kb_newton_F<<<gv, kB, 0, st>>>(M->dev, 0);
-        kb_final<<<g1, kB, 0, st>>>(M->dev, FT_NORM_XK, 0, 0, 0, 0);
+        kb_newton_norm<<<g1, kB, 0, st>>>(M->dev, 0);
         kb_newton_check<<<g1, 32, 0, st>>>(M->dev);
         CKM(cudaGetLastError());
     }
