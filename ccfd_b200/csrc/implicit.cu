@@ -238,7 +238,11 @@ __device__ void fail_member(const ImpDev& d, int status, unsigned devflag) {
     d.ctrl->active = 0;
 }
 
-#define MEMBER const ImpDev& d = I[blockIdx.y]
+// (every kernel of the Newton and Krylov loops is a dependent launch: the
+// vector kernels are a few microseconds each)
+#define MEMBER \
+    grid_wait();  \
+    const ImpDev& d = I[blockIdx.y]
 #define CELL_INDEX                                           \
     if ((int)blockIdx.x >= d.nb) return;                     \
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x
@@ -1141,6 +1145,7 @@ __device__ __forceinline__ bool cluster_compute(const PairSmem<T>& S, const unsi
 template <typename T>
 __global__ void __launch_bounds__(kClThreads) kb_lusgs_cluster(const ImpDev* __restrict__ I, int m) {
     extern __shared__ __align__(16) unsigned char cl_smem[];
+    grid_wait();
     const ImpDev& d = I[blockIdx.x / kClCtas];
     if (!d.precond || !gmres_on(d) || d.fp32 != (sizeof(T) == 4)) return;  // the whole cluster alike
     const int warp = threadIdx.x >> 5, pair = warp >> 1, w = (blockIdx.x % kClCtas) * kClPairs + pair;
@@ -1210,6 +1215,7 @@ __global__ void k_vec_out(int n, const double4* __restrict__ v, const float4* __
 // number of members whose Newton loop is still running
 __global__ void kb_count(const ImpDev* __restrict__ I, int n, int* out) {
     __shared__ int cnt;
+    grid_wait();
     if (threadIdx.x == 0) cnt = 0;
     __syncthreads();
     for (int k = threadIdx.x; k < n; k += blockDim.x)
@@ -1777,15 +1783,15 @@ static void residuals(ImpSet* M, RecKind kind) {
 // same launches), blocks and inverses
 static void build_jacobian(ImpSet* M, cudaStream_t st) {
     const dim3 gv(M->max_nb, M->n);
-    kb_jac_copy<<<gv, kB, 0, st>>>(M->dev);
+    launch_dependent(kb_jac_copy, gv, kB, 0, st, M->dev);
     const dim3 gc((kJacParts * M->max_colsize + 127) / 128, M->n);
-    kb_jac_next<<<gc, 128, 0, st>>>(M->dev, 0);
+    launch_dependent(kb_jac_next, gc, 128, 0, st, M->dev, 0);
     if (M->pc32) residuals(M, REC_JB);
     for (int c = 0; c < M->max_col; ++c) {
         residuals(M, REC_JAC);
-        kb_jac_next<<<gc, 128, 0, st>>>(M->dev, c + 1);
+        launch_dependent(kb_jac_next, gc, 128, 0, st, M->dev, c + 1);
     }
-    kb_jac_finish<<<gv, kB, 0, st>>>(M->dev);
+    launch_dependent(kb_jac_finish, gv, kB, 0, st, M->dev);
 }
 
 // LU-SGS of Krylov vector m of every member, a cluster each.  Two implicit
@@ -1805,12 +1811,14 @@ static int launch_lusgs(ImpSet* M, int m, cudaStream_t st) {
     cfg.blockDim = dim3(kClThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = kClCtas;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kClCtas;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
     CKM(cudaLaunchKernelEx(&cfg, kb_lusgs_cluster<T>, (const ImpDev*)M->dev, m));
     return CCFD_OK;
 }
@@ -1818,7 +1826,7 @@ static int launch_lusgs(ImpSet* M, int m, cudaStream_t st) {
 // members whose Newton loop runs (counted here) / whose GMRES cycle runs
 // (counted by the iteration's kb_givens)
 static int count_on(ImpSet* M, bool newton, int* out) {
-    if (newton) kb_count<<<1, 256, 0, M->stream>>>(M->dev, M->n, M->d_count);
+    if (newton) launch_dependent(kb_count, 1, 256, 0, M->stream, M->dev, M->n, M->d_count);
     CKM(cudaMemcpyAsync(M->h_count, M->d_count, sizeof(int), cudaMemcpyDeviceToHost, M->stream));
     CKM(cudaStreamSynchronize(M->stream));
     *out = *M->h_count;
@@ -1830,47 +1838,47 @@ static int count_on(ImpSet* M, bool newton, int* out) {
 static int set_step(ImpSet* M) {
     cudaStream_t st = M->stream;
     const dim3 gv(M->max_nb, M->n), g1(1, M->n);
-    kb_step_prepare<<<g1, 32, 0, st>>>(M->dev);
-    kb_step_begin<<<gv, kB, 0, st>>>(M->dev);
+    launch_dependent(kb_step_prepare, g1, 32, 0, st, M->dev);
+    launch_dependent(kb_step_begin, gv, kB, 0, st, M->dev);
     residuals(M, REC_NT);
-    kb_newton_F<<<gv, kB, 0, st>>>(M->dev, 1);
-    kb_newton_norm<<<g1, kB, 0, st>>>(M->dev, 1);
-    kb_newton_start<<<g1, 32, 0, st>>>(M->dev);
+    launch_dependent(kb_newton_F, gv, kB, 0, st, M->dev, 1);
+    launch_dependent(kb_newton_norm, g1, kB, 0, st, M->dev, 1);
+    launch_dependent(kb_newton_start, g1, 32, 0, st, M->dev);
     CKM(cudaGetLastError());
     for (int it = 0; it < M->max_newton; ++it) {
         int on = 0, s;
         if ((s = count_on(M, true, &on))) return s;
         if (!on) break;
         // GMRES_M (src/linearSolver.c:385-510)
-        kb_gmres_init<<<gv, kB, 0, st>>>(M->dev);
-        kb_gmres_flags<<<g1, 32, 0, st>>>(M->dev);
+        launch_dependent(kb_gmres_init, gv, kB, 0, st, M->dev);
+        launch_dependent(kb_gmres_flags, g1, 32, 0, st, M->dev);
         if (M->any_precond) {
             build_jacobian(M, st);
-            kb_jac_check<<<g1, 32, 0, st>>>(M->dev);
+            launch_dependent(kb_jac_check, g1, 32, 0, st, M->dev);
         }
         for (int m = 0; m < M->max_K; ++m) {
             if (M->pc64 && (s = launch_lusgs<double>(M, m, st))) return s;
             if (M->pc32 && (s = launch_lusgs<float>(M, m, st))) return s;
-            if (M->any_plain) kb_copy_vz<<<gv, kB, 0, st>>>(M->dev, m);
+            if (M->any_plain) launch_dependent(kb_copy_vz, gv, kB, 0, st, M->dev, m);
             // matrixVector: epsFD = sqrt(eps) / |Z|
-            kb_dot_zz<<<gv, kB, 0, st>>>(M->dev, m, M->d_count);
-            kb_mv_prep<<<gv, kB, 0, st>>>(M->dev, m);
+            launch_dependent(kb_dot_zz, gv, kB, 0, st, M->dev, m, M->d_count);
+            launch_dependent(kb_mv_prep, gv, kB, 0, st, M->dev, m);
             residuals(M, REC_MV);
-            kb_mv_finish<<<gv, kB, 0, st>>>(M->dev, m);
+            launch_dependent(kb_mv_finish, gv, kB, 0, st, M->dev, m);
             // modified Gram-Schmidt
-            for (int nn = 0; nn <= m; ++nn) kb_mgs<<<gv, kB, 0, st>>>(M->dev, nn, m);
-            kb_givens<<<g1, kB, 0, st>>>(M->dev, m, M->d_count);
-            kb_vnext<<<gv, kB, 0, st>>>(M->dev, m);
+            for (int nn = 0; nn <= m; ++nn) launch_dependent(kb_mgs, gv, kB, 0, st, M->dev, nn, m);
+            launch_dependent(kb_givens, g1, kB, 0, st, M->dev, m, M->d_count);
+            launch_dependent(kb_vnext, gv, kB, 0, st, M->dev, m);
             CKM(cudaGetLastError());
             if ((s = count_on(M, false, &on))) return s;
             if (!on) break;
         }
-        kb_gmres_end<<<g1, 32, 0, st>>>(M->dev);
-        kb_newton_update<<<gv, kB, 0, st>>>(M->dev);
+        launch_dependent(kb_gmres_end, g1, 32, 0, st, M->dev);
+        launch_dependent(kb_newton_update, gv, kB, 0, st, M->dev);
         residuals(M, REC_NT);
-        kb_newton_F<<<gv, kB, 0, st>>>(M->dev, 0);
-        kb_newton_norm<<<g1, kB, 0, st>>>(M->dev, 0);
-        kb_newton_check<<<g1, 32, 0, st>>>(M->dev);
+        launch_dependent(kb_newton_F, gv, kB, 0, st, M->dev, 0);
+        launch_dependent(kb_newton_norm, g1, kB, 0, st, M->dev, 0);
+        launch_dependent(kb_newton_check, g1, 32, 0, st, M->dev);
         CKM(cudaGetLastError());
     }
     // global residual of the final residual evaluation, stop tests and the

@@ -71,29 +71,6 @@ struct SmemLimit {
     }
 };
 
-// Launch whose CTAs may be set up while the kernel before it on the stream
-// drains (programmatic dependent launch); they wait in grid_wait(), first
-// thing and on every path, so completion stays in stream order.  Microseconds
-// per stage without / with: 8,000 cells 14.15 / 13.65, 32,761 cells 15.15 /
-// 14.60, 500,000 cells 77.8 / 77.0.  The kernels do not release their
-// dependents early: waiting CTAs then take the slots of running ones (16.6 us
-// at 8,000 cells).
-template <typename... P, typename... A>
-inline void launch_dependent(void (*kern)(P...), int grid, int threads, int smem, cudaStream_t st, const A&... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kern, args...);
-}
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // CTA shapes.  k_grad: 4 / grad_vars threads per cell, at most kGradThreads
 // per CTA.
 // k_flux: at most `threads`, `single` unless the context sets another size.
