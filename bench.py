@@ -160,15 +160,16 @@ def roofline_bytes_per_residual(n_tri: int, n_quad: int, venk: bool) -> int:
             + n_quad * ROOFLINE_BYTES_PER_CELL[("quad", venk)])
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per launch of the
-# stage kernel on this workload from one ncu capture, valid only for the
-# kernel sources whose digest is recorded beside it (STAGE_SOURCES); for
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per stage (one
+# k_grad and one k_flux launch) on this workload from one ncu capture, valid
+# only for the kernel sources whose digest is recorded beside it (STAGE_SOURCES); for
 # other sources the line reports no traffic.
 STAGE_TRAFFIC = {"bytes": 149.260e6 + 8.613e6,
                  "sha256": "c4f694ad24ef324a"}
 STAGE_SOURCES = ("ccfd_b200/csrc/stage_impl.cuh", "ccfd_b200/csrc/physics.cuh",
                  "ccfd_b200/csrc/kernels.cuh", "ccfd_b200/csrc/stage_flux.inc",
-                 "ccfd_b200/csrc/stage_f05.cu", "ccfd_b200/csrc/tiles.cpp")
+                 "ccfd_b200/csrc/stage_f05.cu", "ccfd_b200/csrc/gradients.inc",
+                 "ccfd_b200/csrc/gradients.cu", "ccfd_b200/csrc/tiles.cpp")
 
 
 def stage_sources_digest() -> str:
@@ -748,14 +749,14 @@ def main() -> int:
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak,
                          "unit": "GB/s", "frac": achieved / hbm_peak,
                          "traffic": traffic, "traffic_source": traffic_note,
-                         "kernel": "k_stage: fused residual evaluation + RK stage",
+                         "kernel": "k_grad + k_flux: residual evaluation + RK stage",
                          "bytes_per_launch": bytes_stage,
                          "bytes_per_cell": "364 (two-pass scheme, triangles, Venkatakrishnan)",
                          "fused_bytes_per_launch": bytes_fused, "avg_ms": avg_res_ms,
                          "peak_source": peak_src},
             "e2e": {"value": e2e_value, "unit": UNIT,
                     "h2d_bytes_per_step": n * 4 * 8, "d2h_bytes_per_step": n * 4 * 8},
-            "gpu_launches": int(steps_done * nrk + 2),
+            "gpu_launches": int(steps_done * nrk * 2 + 2),  # k_grad and k_flux per stage
             "clocks": clk,
             "cpu_baseline": cpu,
             "mixed_precision": mixed,

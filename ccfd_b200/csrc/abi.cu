@@ -828,6 +828,7 @@ extern "C" int ccfd_errors(ccfd_ctx* ctx, int exact_func, double out[12]) {
         L.mode = 0;
         L.prim_in = cur_prim(ctx);
         L.grad_out = grad_out_of(ctx);
+        L.ghost_pface = nullptr;  // the wall pressures stay those of the last residual
         launch_gradients(L, ctx->stream);
         CK(cudaGetLastError());
     }

@@ -891,7 +891,7 @@ constexpr int kClSlots = 6;         // chunks whose blocks are in shared memory
 constexpr int kClAhead = 3;         // copies in flight, chunks
 constexpr int kClIdx = 16;          // chunks whose records are in shared memory
 static_assert(kClIdx >= kClSlots + 2 * kClAhead + 1, "a record outlives its blocks");
-constexpr int kClSpin = 1 << 20;    // polls before the sweep gives up
+constexpr int kClSpin = 1 << 25;    // polls (~60 cycles each, about a second) before the sweep gives up
 
 // One place of a chunk: cell (-1: none), half-sides of its blocks in side
 // order (-1: none), where the neighbours' values are and where its own result
