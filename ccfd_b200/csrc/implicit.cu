@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(128) kb_jac_next(const ImpDev* __restrict__ I,
         if (e < 0) return;
         t = 16 * (long)d.twin[h];
     }
-    const double sreps = 1.0 / reps;
+    const double sreps = 1.0 / reps, dt = d.ctrl->dt;
     double r[4], u[4][4];
     ld(d.fp32 ? d.rjb[e] : d.RXK[e], r);
 #pragma unroll
@@ -641,11 +641,22 @@ __global__ void __launch_bounds__(128) kb_jac_next(const ImpDev* __restrict__ I,
         double o[4];
 #pragma unroll
         for (int v = 0; v < 4; ++v) o[v] = 0.0 + (u[v][j] - r[j]) * sreps;
-        if (part == 0) *reinterpret_cast<double4*>(d.D + t + 4 * j) = mk(o);
-        else if (d.fp32)
-            *reinterpret_cast<float4*>(d.Of + t + 4 * j) =
-                make_float4((float)o[0], (float)o[1], (float)o[2], (float)o[3]);
-        else *reinterpret_cast<double4*>(d.O + t + 4 * j) = mk(o);
+        if (part == 0) {
+            *reinterpret_cast<double4*>(d.D + t + 4 * j) = mk(o);
+            continue;
+        }
+        // the off-diagonal blocks of I - dt J (src/linearSolver.c:226-234);
+        // the FP32 blocks are rounded before and after the scaling
+        if (d.fp32) {
+            float f[4];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) f[v] = (float)((double)(float)o[v] * -dt);
+            *reinterpret_cast<float4*>(d.Of + t + 4 * j) = make_float4(f[0], f[1], f[2], f[3]);
+        } else {
+#pragma unroll
+            for (int v = 0; v < 4; ++v) o[v] = o[v] * -dt;
+            *reinterpret_cast<double4*>(d.O + t + 4 * j) = mk(o);
+        }
     }
 }
 
@@ -686,7 +697,8 @@ __device__ bool inv4(const double a[16], double r[16]) {
     return true;
 }
 
-// I - dt J on the stored blocks and the inverses of the diagonal blocks
+// I - dt J on the diagonal blocks and their inverses (kb_jac_next has scaled
+// the off-diagonal ones: a pass over them took two thirds of this kernel)
 // (src/linearSolver.c:226-251)
 __global__ void kb_jac_finish(const ImpDev* __restrict__ I) {
     MEMBER;
@@ -709,15 +721,9 @@ __global__ void kb_jac_finish(const ImpDev* __restrict__ I) {
     if (d.fp32) {
 #pragma unroll
         for (int k = 0; k < 16; ++k) d.Dinvf[16 * i + k] = (float)r[k];
-        for (long h = d.hs_off[i]; h < d.hs_off[i + 1]; ++h)
-#pragma unroll
-            for (int k = 0; k < 16; ++k) d.Of[16 * h + k] = (float)((double)d.Of[16 * h + k] * -dt);
     } else {
 #pragma unroll
         for (int k = 0; k < 16; ++k) d.Dinv[16 * i + k] = r[k];
-        for (long h = d.hs_off[i]; h < d.hs_off[i + 1]; ++h)
-#pragma unroll
-            for (int k = 0; k < 16; ++k) d.O[16 * h + k] = d.O[16 * h + k] * -dt;
     }
 }
 
