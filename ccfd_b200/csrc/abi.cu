@@ -964,8 +964,8 @@ extern "C" int ccfd_get_history(ccfd_ctx* ctx, double* rows, long max_rows, long
     return CCFD_OK;
 }
 
-// Autotuner of the stage kernel's launch shape: cells per tile (which sets
-// the CTA's faces and gradient cells per thread) and the cell ordering
+// Autotuner of the flux kernel's launch shape: cells per tile (which sets
+// the CTA's cells and faces per thread) and the cell ordering
 // (Hilbert curve or the reference's numbering).  Every candidate is uploaded
 // and timed over a few residual evaluations of the given state; the context
 // keeps the fastest.  Results do not depend on the choice (the arithmetic

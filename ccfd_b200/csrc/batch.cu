@@ -2,8 +2,8 @@
 //
 // Every member is an ordinary context (its own mesh, state, control block and
 // scratch, all resident in device memory).  Explicit members are advanced
-// together: each Runge-Kutta stage is one launch per kernel variant (flux,
-// order, equations, precision) over the concatenated tiles of all members of
+// together: each Runge-Kutta stage is one launch pair per kernel variant
+// (flux, order, equations, precision) over the concatenated tiles of all members of
 // that variant, so small and uneven meshes fill the GPU together.  Each
 // member keeps its own time step, CFL, stop tests and convergence flags in
 // its control block; a member that stops simply returns from its CTAs.  A

@@ -19,7 +19,7 @@ struct ccfd_ctx {
     ccfd::TileDev tiles;
     ccfd::GhostDev ghosts;
     int tile_cells = 0;     // cells per tile, 0: by the mesh size
-    int stage_threads = 0;  // CTA size of the stage kernel, 0: the precision's default
+    int stage_threads = 0;  // CTA size of the flux kernel, 0: the precision's default
     ccfd_exact exact;
     double rk[6];
     double total_area_q = 0.0;

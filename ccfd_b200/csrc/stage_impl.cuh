@@ -33,9 +33,10 @@
 // warps per SM, ring cells computed twice, half the threads idle in the
 // second pass of each phase.  The split keeps each loop's registers low
 // enough for 28 warps, computes every gradient once and streams the face
-// states: 76, 167 and 14 us (64 us with FP32 fluxes), at 0.13 GB of DRAM
-// traffic per kernel.  Both are bound by memory latency (the scheduler
-// issues in ~45 % of its cycles) and by correctly rounded FP64 divisions.
+// states: 76, 167 and 13.7 us (62 us with FP32 fluxes), at 0.13 + 0.12 GB of
+// DRAM traffic on the 500,000 triangles.  Both kernels are bound by memory
+// latency (the scheduler issues in ~42 % of its cycles) and by chains of
+// correctly rounded FP64 divisions.
 //
 // Floating-point operations keep the reference's operand order; the FP64
 // units are compiled with -fmad=false, so their results equal the reference's.
@@ -74,7 +75,9 @@ struct SmemLimit {
 // CTA shapes.  k_grad: 4 / grad_vars threads per cell, at most kGradThreads
 // per CTA.
 // k_flux: at most `threads`, `single` unless the context sets another size.
-// regs / regs_ns (viscous) / grad_regs cap the registers per thread.
+// regs / regs_ns (viscous) / grad_regs cap the registers per thread: 76 us per
+// stage (500,000 triangles) at 72 registers in k_grad, 84 at 80, 82 at 64 and
+// 96; viscous flux 48.9 us (200,000 triangles) at 128, 50.0 at 112, 52.3 at 96.
 constexpr int kGradThreads = 128;
 template <typename FT> struct StageShape;
 template <> struct StageShape<double> { static constexpr int threads = 384, single = 128, regs = 72, regs_ns = 128, grad_vars = 2, grad_regs = 72; };
@@ -174,11 +177,6 @@ template <typename T>
 __device__ __forceinline__ typename Vec<T>::v4 cvt4(const double4& v) {
     if constexpr (sizeof(T) == 8) return v;
     else return make_float4(float(v.x), float(v.y), float(v.z), float(v.w));
-}
-template <typename T>
-__device__ __forceinline__ typename Vec<T>::v2 cvt2(double a, double b) {
-    if constexpr (sizeof(T) == 8) return make_double2(a, b);
-    else return make_float2(float(a), float(b));
 }
 __device__ __forceinline__ double4 to_d4(const double4& v) { return v; }
 __device__ __forceinline__ double4 to_d4(const float4& v) {

@@ -1,5 +1,5 @@
 // Hilbert ordering of cells and construction of the staged tiles of the
-// fused stage kernel (see tiles.h).
+// stage kernels (see tiles.h).
 #include "tiles.h"
 
 #include <algorithm>

@@ -391,11 +391,11 @@ int ccfd_write_history(const ccfd_case *c, const double *rows, long n_rows, int 
 int ccfd_errors(ccfd_ctx *ctx, int exact_func, double out[12]);
 
 /* Autotuner (no counterpart in the reference): re-uploads the case with
- * each candidate launch shape of the stage kernel (cells per tile 128..384,
+ * each candidate launch shape of the stage kernels (cells per tile 128..384,
  * Hilbert or reference cell order) and times residual evaluations of state
  * prim ([n_cells][4] primitive, reference order) at each CTA size (FP64
  * 256 / 320 / 384 threads, FP32 fluxes 128 / 192 / 256, so cells and faces
- * per thread vary with the tile), keeps the fastest; the context ends
+ * per thread of the flux kernel vary with the tile), keeps the fastest; the context ends
  * uploaded with that shape and with prim as its state.  Results are
  * independent of the shape.  Outputs may be NULL. */
 int ccfd_autotune(ccfd_ctx *ctx, const ccfd_mesh *m, const ccfd_bc *bc, int n_bc,
@@ -427,7 +427,7 @@ int ccfd_exact_state(ccfd_ctx *ctx, int exact_func, double time, double *prim_ou
  * ccfd_set_state, ccfd_residual and ccfd_set_time return CCFD_ERR_BUSY,
  * ccfd_get_state and ccfd_batch_report read its current state and control
  * block.  Explicit members advance in multi-instance stage launches over
- * their concatenated tiles (one launch per kernel variant and RK stage,
+ * their concatenated tiles (one gradient and one flux launch per kernel variant and RK stage,
  * replayed from a CUDA graph); implicit members advance in lockstep Newton /
  * GMRES / LU-SGS iterations whose kernels cover every member at once.  Each
  * member keeps its own time step, CFL, stop criteria and flags. */
