@@ -249,10 +249,11 @@ static void par_for(long n, Fn fn) {
 
 // Cells per tile when the context sets none.  A large tile repeats fewer
 // border faces, a small one leaves fewer SMs idle: microseconds per RK stage
-// at 48 / 64 / 128 / 256 cells (HLLC, 128 threads): 8,000 cells 13.7 / 15.5 /
-// 18.9 / 26.8, 32,761 cells 14.9 / 15.8 / 19.1 / 27.2, 62,834 cells 23.4 /
-// 20.3 / 20.8 / 27.1, 130,321 cells 35.1 / 33.2 / 31.9 / 32.7; at 128 / 256:
-// 500,000 cells 83.1 / 81.3, 1,048,576 cells 185.6 / 175.1.
+// at 48 / 64 / 128 / 256 cells (HLLC, 128 threads): 8,000 cells 13.7 / 15.0 /
+// 18.7 / 26.9, 32,761 cells 14.5 / 15.2 / 18.6 / 26.5, 62,834 cells 22.1 /
+// 18.0 / 19.9 / 26.2, 130,321 cells 35.0 / 31.9 / 27.2 / 32.6; at 128 / 256:
+// 500,000 cells 78.9 / 76.1, 1,048,576 cells 175 / 167, viscous 200,000 cells
+// 49.9 / 54.0.
 static int default_tile_cells(long n) { return n < 48000 ? 48 : n < 96000 ? 64 : n < 320000 ? 128 : 256; }
 
 // Host staging of an upload, kept per thread from one upload to the next:
