@@ -104,8 +104,11 @@ __device__ __forceinline__ float4 mk4(const float q[4]) {
 
 // One 32-byte record per load / store instruction (256-bit accesses; the
 // records are 32-byte aligned): a gather then costs one request and one tag
-// lookup per sector instead of two.  ld32 is for data the kernel does not
-// write; ld32_rw keeps its place among the kernel's stores.
+// lookup per sector instead of two.  ld32 is for mesh records, which nothing
+// writes while kernels run: to the compiler it is a pure function of the
+// address.  What kernels write, this one or the one before it, is loaded by
+// ld32_rw and the volatile loads below, which keep their place behind
+// grid_wait(), barriers and stores.
 __device__ __forceinline__ double4 ld32(const double4* p) {
     double4 v;
     asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
@@ -146,24 +149,26 @@ __device__ __forceinline__ void ld_rw(const double* p, double (&v)[2]) {
 // The gradients of a cell are stored variable by variable, (x0, y0, x1, y1),
 // (x2, y2, x3, y3), as the threads of the cell write them.
 __device__ __forceinline__ void ld_grad(const double4* p, double gx[4], double gy[4]) {
-    const double4 a = ld32(p), b = ld32(p + 1);
+    const double4 a = ld32_rw(p), b = ld32_rw(p + 1);
     gx[0] = a.x; gy[0] = a.y; gx[1] = a.z; gy[1] = a.w;
     gx[2] = b.x; gy[2] = b.y; gx[3] = b.z; gy[3] = b.w;
 }
 __device__ __forceinline__ void ld_grad(const float4* p, float gx[4], float gy[4]) {
-    asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(gx[0]), "=f"(gy[0]), "=f"(gx[1]), "=f"(gy[1]), "=f"(gx[2]), "=f"(gy[2]), "=f"(gx[3]), "=f"(gy[3])
-        : "l"(p));
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(gx[0]), "=f"(gy[0]), "=f"(gx[1]), "=f"(gy[1]), "=f"(gx[2]), "=f"(gy[2]), "=f"(gx[3]), "=f"(gy[3])
+                 : "l"(p)
+                 : "memory");
 }
 // the two reconstructed states of a face
 __device__ __forceinline__ void ld_face(const double4* p, double l[4], double r[4]) {
-    ld4(ld32(p), l);
-    ld4(ld32(p + 1), r);
+    ld4(ld32_rw(p), l);
+    ld4(ld32_rw(p + 1), r);
 }
 __device__ __forceinline__ void ld_face(const float4* p, float l[4], float r[4]) {
-    asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(l[0]), "=f"(l[1]), "=f"(l[2]), "=f"(l[3]), "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3])
-        : "l"(p));
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(l[0]), "=f"(l[1]), "=f"(l[2]), "=f"(l[3]), "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3])
+                 : "l"(p)
+                 : "memory");
 }
 
 // shared-memory vector types of the stage kernel: FP64 throughout, or FP32
@@ -808,9 +813,9 @@ __device__ __forceinline__ void flux_body(const StageLaunch& L, const int t) {
             const int2 lr = face_cells(nl);
             const bool inner = lr.y >= 0;
             if (NS) bb = ld32_once(T.f_bb + id);
-            ld4(cvt4<FT>(ld32(L.prim_in + lr.x)), q0);
-            if (inner) ld4(cvt4<FT>(ld32(L.prim_in + lr.y)), q1);
-            else if (ORDER == 2) ld4(cvt4<FT>(ld32(L.ghosts.state + (-1 - lr.y))), q1);
+            ld4(cvt4<FT>(ld32_rw(L.prim_in + lr.x)), q0);
+            if (inner) ld4(cvt4<FT>(ld32_rw(L.prim_in + lr.y)), q1);
+            else if (ORDER == 2) ld4(cvt4<FT>(ld32_rw(L.ghosts.state + (-1 - lr.y))), q1);
             if (ORDER == 2) {
                 const V4* grad = reinterpret_cast<const V4*>(L.grad);
                 const double4 gp = ld32_once(T.f_gp + id);
