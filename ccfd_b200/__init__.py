@@ -274,9 +274,10 @@ class Solver:
         return ms.value, cnt.value
 
     def autotune(self, state: np.ndarray | None = None) -> dict:
-        """Pick the stage kernel's tile size, cell ordering and CTA size by
-        timing (ccfd_autotune); the solver keeps the fastest and `state`
-        (default: the case's initial state)."""
+        """Pick the stage kernels' tile size, cell ordering and CTA size by
+        timing (ccfd_autotune); the solver keeps the fastest shape, its own
+        included, and `state` (default: the case's initial state).  Returns
+        the fastest candidate."""
         c = self.case.c
         prim = np.ascontiguousarray(self.case.prim0() if state is None else state,
                                     dtype=np.float64).reshape(self.n, 4)

@@ -390,14 +390,15 @@ int ccfd_write_history(const ccfd_case *c, const double *rows, long n_rows, int 
  * buffer (stream-ordered). */
 int ccfd_errors(ccfd_ctx *ctx, int exact_func, double out[12]);
 
-/* Autotuner (no counterpart in the reference): re-uploads the case with
- * each candidate launch shape of the stage kernels (cells per tile 128..384,
- * Hilbert or reference cell order) and times residual evaluations of state
- * prim ([n_cells][4] primitive, reference order) at each CTA size (FP64
- * 256 / 320 / 384 threads, FP32 fluxes 128 / 192 / 256, so cells and faces
- * per thread of the flux kernel vary with the tile), keeps the fastest; the context ends
- * uploaded with that shape and with prim as its state.  Results are
- * independent of the shape.  Outputs may be NULL. */
+/* Autotuner (no counterpart in the reference): times residual evaluations of
+ * state prim ([n_cells][4] primitive, reference order) with the context's own
+ * launch shape (on the Hilbert curve) and with each candidate of the stage
+ * kernels, re-uploading the case: cells per tile 128..384, Hilbert or
+ * reference cell order, CTA size (FP64 256 / 320 / 384 threads, FP32 fluxes
+ * 128 / 192 / 256, so cells and faces per thread of the flux kernel vary with
+ * the tile).  The context ends uploaded with the fastest of all, its own
+ * included, and with prim as its state; the outputs describe the fastest
+ * candidate.  Results are independent of the shape.  Outputs may be NULL. */
 int ccfd_autotune(ccfd_ctx *ctx, const ccfd_mesh *m, const ccfd_bc *bc, int n_bc,
 		  const ccfd_exact *ex, const double *prim, int *tile_cells, int *reorder,
 		  int *threads, double *ms_per_residual);
