@@ -1377,7 +1377,9 @@ int ccfd_implicit_setup(ccfd_ctx* ctx, const std::vector<int>& hs_off, const std
         std::vector<int> fill(coff.begin(), coff.end() - 1);
         for (long d = 0; d < N; ++d) ccells[fill[color[d]]++] = (int)d;
         S->color_off = coff;
-        // lower / upper neighbour lists in side order, by reference number
+        // lower / upper neighbour lists in side order, by reference number; a
+        // cell that is its own neighbour (a periodic mesh one cell wide) is in
+        // neither, as in the reference's loops (src/linearSolver.c:261-333)
         const std::vector<int>& ref = ctx->cell_of_dev;
         std::vector<int> lo_off(N + 1, 0), up_off(N + 1, 0), lo_nb, lo_h, up_nb, up_h;
         for (long d = 0; d < N; ++d) {
@@ -1385,7 +1387,7 @@ int ccfd_implicit_setup(ccfd_ctx* ctx, const std::vector<int>& hs_off, const std
             up_off[d] = (int)up_nb.size();
             for (int h = hs_off[d]; h < hs_off[d + 1]; ++h) {
                 int e = hs_nb[h];
-                if (e < 0) continue;
+                if (e < 0 || e == d) continue;
                 if (ref[e] < ref[d]) {
                     lo_nb.push_back(e);
                     lo_h.push_back(h);
