@@ -1540,6 +1540,10 @@ int ccfd_implicit_setup(ccfd_ctx* ctx, const std::vector<int>& hs_off, const std
             (st = iupload(ctx, &S->bw_nb, bwn)) || (st = iupload(ctx, &S->bw_h, bwh)))
             return st;
     }
+    // a block that no column is recorded in (boundary sides; on a periodic mesh
+    // two cells wide the second side of a pair of cells) is zero
+    if (S->Of) CK(cudaMemsetAsync(S->Of, 0, sizeof(float) * 16 * (size_t)H, ctx->stream));
+    if (S->O) CK(cudaMemsetAsync(S->O, 0, sizeof(double) * 16 * (size_t)H, ctx->stream));
     CK(cudaMemsetAsync(S->sc, 0, sizeof(double) * (SC_H + (K + 1) * (K + 1) + 4 * (K + 1) + 8), ctx->stream));
     CK(cudaMemsetAsync(S->flag, 0, sizeof(int) * 8, ctx->stream));
     CK(cudaMemsetAsync(S->ctl, 0, sizeof(int) * CTL_WORDS, ctx->stream));
