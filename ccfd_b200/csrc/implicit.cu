@@ -1574,7 +1574,7 @@ struct ImpSet {
     int max_level = 0;  // widest LU-SGS level (cells) over the members
     bool any_precond = false;
     bool any_plain = false;  // a member without preconditioner
-    bool cluster = false;  // LU-SGS by clusters
+    bool cluster = false;  // LU-SGS by clusters (every preconditioned member fits)
     bool pc64 = false, pc32 = false;  // preconditioned members in FP64 / FP32
     int* d_count = nullptr;
     int* h_count = nullptr;
@@ -1652,6 +1652,11 @@ static ImpDev make_dev(ccfd_ctx* ctx) {
     return d;
 }
 
+// the member's sweeps, if it has any, fit the cluster kernel
+static bool sweeps_by_cluster(const ccfd_ctx* ctx) {
+    return !ctx->params.precond || ((const ImpState*)ctx->implicit_state)->cluster_ok;
+}
+
 static int set_build(const std::vector<ccfd_ctx*>& members, cudaStream_t stream, ImpSet** out) {
     ImpSet* M = new ImpSet();
     *out = M;
@@ -1659,7 +1664,7 @@ static int set_build(const std::vector<ccfd_ctx*>& members, cudaStream_t stream,
     M->n = (int)members.size();
     M->stream = stream;
     M->cluster = true;
-    for (ccfd_ctx* ctx : members) M->cluster = M->cluster && ((ImpState*)ctx->implicit_state)->cluster_ok;
+    for (ccfd_ctx* ctx : members) M->cluster = M->cluster && sweeps_by_cluster(ctx);
     if (M->cluster) {
         CKM(cudaFuncSetAttribute(kb_lusgs_cluster<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  cluster_smem<double>()));
@@ -1819,8 +1824,8 @@ static void build_jacobian(ImpSet* M, cudaStream_t st) {
 // LU-SGS of Krylov vector m of every member, a cluster each.  Two implicit
 // steps of the first n airfoils of the batched set took, with clusters / one
 // CTA per member (ms): n = 16 84 / 180, 32 114 / 196, 64 190 / 273, 128 384 /
-// 526; one CTA per member is left to numberings that need more mailboxes than
-// a CTA has.
+// 526; one CTA per member is left to sets with a numbering that needs more
+// mailboxes than a CTA has.
 template <typename T>
 static int launch_lusgs(ImpSet* M, int m, cudaStream_t st) {
     if (!M->cluster) {
@@ -2195,20 +2200,33 @@ int ccfd_implicit_batch_steps(ccfd_batch* b, const std::vector<ccfd_ctx*>& membe
         // sets balanced by cell count (largest first onto the lightest set);
         // at most CCFD_IMPLICIT_SETS (default 8) sets of at least 4 members
         // (256 airfoils: 2 / 4 / 8 / 16 sets 3.17 / 2.93 / 2.75 / 2.87 s;
-        // 32 airfoils: 4 and 8 sets alike)
+        // 32 airfoils: 4 and 8 sets alike).  Members whose sweeps need the
+        // single-CTA kernel get sets of their own, since a set sweeps by one
+        // kernel: eight airfoils, one of them with a shuffled numbering, took
+        // 30.0 ms for three steps in one set, 17.0 in two.
         int max_sets = 8;
         if (const char* e = getenv("CCFD_IMPLICIT_SETS")) max_sets = std::max(1, std::min(64, atoi(e)));
-        const int nsets = std::max(1, std::min(max_sets, (int)members.size() / 4));
-        std::vector<int> idx(members.size());
-        for (size_t k = 0; k < idx.size(); ++k) idx[k] = (int)k;
-        std::stable_sort(idx.begin(), idx.end(), [&](int a, int c) { return members[a]->N > members[c]->N; });
-        std::vector<std::vector<ccfd_ctx*>> parts(nsets);
-        std::vector<long> load(nsets, 0);
-        for (int k : idx) {
-            int j = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-            parts[j].push_back(members[k]);
-            load[j] += members[k]->N;
+        std::vector<int> idx[2];  // by route: any kernel will do or clusters, one CTA
+        for (size_t k = 0; k < members.size(); ++k)
+            idx[max_sets > 1 && !sweeps_by_cluster(members[k])].push_back((int)k);
+        std::vector<std::vector<ccfd_ctx*>> parts;
+        int left = max_sets;
+        for (int r = 1; r >= 0; --r) {
+            if (idx[r].empty()) continue;
+            const int most = r && !idx[0].empty() ? left - 1 : left;
+            const int n = std::max(1, std::min(most, (int)idx[r].size() / 4));
+            left -= n;
+            std::stable_sort(idx[r].begin(), idx[r].end(), [&](int a, int c) { return members[a]->N > members[c]->N; });
+            const size_t first = parts.size();
+            parts.resize(first + n);
+            std::vector<long> load(n, 0);
+            for (int k : idx[r]) {
+                const int j = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+                parts[first + j].push_back(members[k]);
+                load[j] += members[k]->N;
+            }
         }
+        const int nsets = (int)parts.size();
         for (int j = 0; j < nsets; ++j) {
             cudaStream_t st;
             if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return CCFD_ERR_CUDA;
