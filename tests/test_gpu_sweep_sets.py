@@ -91,3 +91,25 @@ def test_not_finite_values_arrive(precision, bits):
     want = restated.lusgs(case, Di, O, rhs)
     assert np.array_equal(np.isnan(x), np.isnan(want))
     assert np.isnan(x).any()
+
+
+# levels of several chunks and ranges that cut rows, in FP32 by clusters, and by
+# one CTA on the shuffled numbering
+@pytest.mark.parametrize("ni,nj,kind", [(70, 40, "fits"), (33, 32, "fits"), (128, 100, "shuffled")])
+def test_fp32_sweep_matches_the_oracle(ni, nj, kind):
+    from oracle import restated
+    case = _airfoil(ni, nj, kind, precision=1)
+    s = cc.Solver(case)
+    _, Di, O = s.build_matrix(0.0, 0.05 * s.calc_time_step())
+    rhs = np.random.Generator(np.random.PCG64(17)).standard_normal((case.n_cells, 4))
+    rhs = rhs.astype(np.float32).astype(np.float64)
+    x = s.lusgs(rhs)
+    s.close()
+    # some 60 rounded operations a row; a row passes its error on by the factor
+    # |D^-1 O| summed over its sides, below 1/2 at this time step: two sweeps
+    # stay below 2 * 2 * 60 * 2^-24 < 1.5e-5
+    off = case.mesh()["hs_offset"][:-1]
+    across = np.add.reduceat(np.abs(O).sum(axis=2).max(axis=1), off)
+    assert (across * np.abs(Di).sum(axis=2).max(axis=1)).max() < 0.5
+    want = restated.lusgs(case, Di, O, rhs)
+    assert np.abs(x - want).max() <= 1.5e-5 * np.abs(want).max()
