@@ -180,11 +180,11 @@ __device__ __forceinline__ void block_partial(double v, double* partial) {
 }
 
 // Sum of a member's nb block partials, the same in every block that asks for
-// it (kB threads, fixed order): the kernel that needs a dot product finishes
-// it itself instead of waiting for a launch in between.
+// it (kB threads, fixed order).
 __device__ __forceinline__ double block_total(const double* partial, int nb) {
     __shared__ double sh[kB];
     double v = 0.0;
+#pragma unroll 8
     for (int k = threadIdx.x; k < nb; k += kB) v += partial[k];
     sh[threadIdx.x] = v;
     __syncthreads();
@@ -195,6 +195,19 @@ __device__ __forceinline__ double block_total(const double* partial, int nb) {
     const double r = sh[0];
     __syncthreads();
     return r;
+}
+
+// A dot product in the kernel that needs it: up to kFusedParts partials are
+// summed there by every block, instead of waiting for a launch in between;
+// kb_total leaves the sum of more behind them (what every block reads grows
+// with the square of the mesh).  Milliseconds of an
+// unpreconditioned step of 12 to 16 Krylov iterations, summed in the consumers /
+// by kb_total: 32,768 cells 1.61 / 1.96, 131,072 2.05 / 2.20, 262,144 2.89 /
+// 3.15, 524,288 (2,048 partials) 4.13 / 4.12, 1,048,576 7.08 / 6.75, 2,097,152
+// 13.7 / 12.6, 4,194,304 26.4 / 21.3.
+constexpr int kFusedParts = 2048;
+__device__ __forceinline__ double dot_total(const double* partial, int nb) {
+    return nb > kFusedParts ? partial[nb] : block_total(partial, nb);
 }
 
 // Krylov basis access in the member's precision (FP64 arithmetic outside)
@@ -369,6 +382,15 @@ __global__ void kb_copy_vz(const ImpDev* __restrict__ I, int m) {
     if (i < d.N) putZ(d, (long)m * d.N + i, getV(d, (long)m * d.N + i));
 }
 
+// sums of more than kFusedParts partials of buffer `buf`, left behind them
+__global__ void kb_total(const ImpDev* __restrict__ I, int buf) {
+    MEMBER;
+    if (d.nb <= kFusedParts || !gmres_on(d)) return;
+    double* const partial = d.partial + buf * (d.nb + 1);
+    const double r = block_total(partial, d.nb);
+    if (threadIdx.x == 0) partial[d.nb] = r;
+}
+
 // |Z_m|^2 partials; also clears the count of members that iterate on
 // (kb_givens counts them)
 __global__ void kb_dot_zz(const ImpDev* __restrict__ I, int m, int* count) {
@@ -390,7 +412,7 @@ __global__ void kb_mv_prep(const ImpDev* __restrict__ I, int m) {
     MEMBER;
     if (!gmres_on(d)) return;
     CELL_INDEX;
-    const double e = sqrt(DBL_EPSILON) / sqrt(block_total(d.partial, d.nb));
+    const double e = sqrt(DBL_EPSILON) / sqrt(dot_total(d.partial, d.nb));
     if (i == 0) d.sc[SC_EPSFD] = e;
     if (i >= d.N) return;
     double x[4], z[4], c[4], p[4];
@@ -428,16 +450,15 @@ __global__ void kb_mv_finish(const ImpDev* __restrict__ I, int m) {
 // H[nn][m] from the partials of V_nn . W; W -= H[nn][m] V_nn (modified
 // Gram-Schmidt step, src/linearSolver.c:440-450), then the partial of
 // V_{nn+1} . W (or W . W after the last one) into the other partial buffer
-// (a member's later blocks may still read this one).  Every block sums the
-// previous kernel's partials itself, in the same order: a launch in between for
-// the sum took 4.6 us of the pair's 10.1 on 32,768 cells, this one takes 6.7.
+// (a member's later blocks may still read this one).  On 32,768 cells a launch
+// in between for the sum took 4.6 us of the pair's 10.1, this one takes 6.7.
 __global__ void kb_mgs(const ImpDev* __restrict__ I, int nn, int m) {
     MEMBER;
     if (!gmres_on(d)) return;
     CELL_INDEX;
     double* const in = d.partial + (nn & 1) * (d.nb + 1);
     double* const out = d.partial + ((nn + 1) & 1) * (d.nb + 1);
-    const double hh = block_total(in, d.nb);
+    const double hh = dot_total(in, d.nb);
     if (i == 0) d.sc[SC_H + nn * (d.K + 1) + m] = hh;
     double dd = 0.0;
     if (i < d.N) {
@@ -1889,11 +1910,16 @@ static int set_step(ImpSet* M) {
             if (M->any_plain) launch_dependent(kb_copy_vz, gv, kB, 0, st, M->dev, m);
             // matrixVector: epsFD = sqrt(eps) / |Z|
             launch_dependent(kb_dot_zz, gv, kB, 0, st, M->dev, m, M->d_count);
+            const bool sums = M->max_nb > kFusedParts;
+            if (sums) launch_dependent(kb_total, g1, kB, 0, st, M->dev, 0);
             launch_dependent(kb_mv_prep, gv, kB, 0, st, M->dev, m);
             residuals(M, REC_MV);
             launch_dependent(kb_mv_finish, gv, kB, 0, st, M->dev, m);
             // modified Gram-Schmidt
-            for (int nn = 0; nn <= m; ++nn) launch_dependent(kb_mgs, gv, kB, 0, st, M->dev, nn, m);
+            for (int nn = 0; nn <= m; ++nn) {
+                if (sums) launch_dependent(kb_total, g1, kB, 0, st, M->dev, nn & 1);
+                launch_dependent(kb_mgs, gv, kB, 0, st, M->dev, nn, m);
+            }
             launch_dependent(kb_givens, g1, kB, 0, st, M->dev, m, M->d_count);
             launch_dependent(kb_vnext, gv, kB, 0, st, M->dev, m);
             CKM(cudaGetLastError());
