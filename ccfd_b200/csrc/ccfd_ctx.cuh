@@ -97,4 +97,6 @@ int ccfd_residual_of(ccfd_ctx* ctx, const double4* prim, double time, double4* u
 // implicit solver set-up / release (implicit.cu); the device buffers are
 // owned by the context's allocation list
 int ccfd_implicit_setup(ccfd_ctx* ctx, const std::vector<int>& hs_off, const std::vector<int>& hs_nb);
+// device bytes that it will take
+size_t ccfd_implicit_bytes(const ccfd_params* p, const ccfd_mesh* m);
 void ccfd_implicit_free(ccfd_ctx* ctx);

@@ -1305,6 +1305,71 @@ void ccfd_implicit_free(ccfd_ctx* ctx) {
     ctx->implicit_state = nullptr;
 }
 
+// Records of one cluster sweep: places of the workers' chunks of up to eight
+// cells of one level (the same for every cell order on the device); 0 where the
+// chunks stay so empty that the sweep is left to the single-CTA kernel.
+static long sweep_records(const ccfd_mesh* m, bool fwd) {
+    const long N = m->n_cells;
+    std::vector<int> lev(N, 0), cnt;
+    int nl = 1;
+    for (long k = 0; k < N; ++k) {
+        const long i = fwd ? k : N - 1 - k;
+        int l = 0;
+        for (long h = m->hs_offset[i]; h < m->hs_offset[i + 1]; ++h) {
+            const long e = m->hs_nb[h];
+            if (e >= 0 && (fwd ? e < i : e > i)) l = std::max(l, lev[e] + 1);
+        }
+        lev[i] = l;
+        nl = std::max(nl, l + 1);
+    }
+    cnt.assign(nl, 0);
+    long chunks = 0;
+    for (long first = 0, last; first < N; first = last) {
+        const long w = first * kClWorkers / N;
+        for (last = first; last < N && last * kClWorkers / N == w; ++last) ++cnt[lev[last]];
+        for (long i = first; i < last; ++i) {
+            chunks += (cnt[lev[i]] + 7) / 8;
+            cnt[lev[i]] = 0;
+        }
+    }
+    return 8 * chunks > 4 * N + kClSpareRecs ? 0 : 8 * chunks;
+}
+
+// Device bytes of ccfd_implicit_setup, array by array as it allocates them
+// (the column scratch by the same first fit into the idle Krylov vectors).
+size_t ccfd_implicit_bytes(const ccfd_params* p, const ccfd_mesh* m) {
+    const size_t N = m->n_cells, H = m->n_half_sides, F = m->n_faces, B = m->n_bc;
+    const size_t K = std::max(1, p->n_kdim), nb = (N + kB - 1) / kB;
+    const bool fp32 = p->precision == CCFD_MIXED;
+    const size_t vec = fp32 ? sizeof(float4) : sizeof(double4), word = fp32 ? sizeof(float) : sizeof(double);
+    size_t b = vec * (2 * K + 1) * N + 8 * sizeof(double4) * N;
+    b += sizeof(double) * (SC_H + (K + 1) * (K + 1) + 4 * (K + 1) + 8 + 2 * (nb + 1)) + 4 * (8 + CTL_WORDS);
+    if (!p->precond) return b;
+    // D, D^-1, off-diagonal blocks, sweep vector, base of the FP32 columns
+    b += sizeof(double) * 16 * N + word * 16 * (N + H) + vec * N + (fp32 ? sizeof(double4) * N : 0);
+    size_t left[2] = {vec * K * N, vec * K * N};
+    auto take = [&](size_t bytes) {
+        for (size_t& l : left)
+            if (bytes + 256 <= l) {
+                l -= bytes + 256;
+                return;
+            }
+        b += bytes;
+    };
+    for (int v = 0; v < 4; ++v) {
+        take(sizeof(double4) * N);
+        take(sizeof(double4) * N);
+        if (p->spatial_order == 2) take(2 * vec * (p->eqn == CCFD_NAVIER_STOKES ? N : F));
+        b += sizeof(double4) * 2 * (B + 1);
+    }
+    // twins, colours (cells, offsets), levels (cells, neighbours, half-sides,
+    // offsets: at most one level per cell), cluster sequences
+    b += sizeof(int) * (H + 2 * N) + 2 * (sizeof(int) * 2 + 2 * sizeof(int4)) * N;
+    const long fw = sweep_records(m, true), bw = sweep_records(m, false);
+    if (fw && bw) b += sizeof(SweepRec) * (fw + bw) + sizeof(int) * 2 * (kClWorkers + 1);
+    return b;
+}
+
 int ccfd_implicit_setup(ccfd_ctx* ctx, const std::vector<int>& hs_off, const std::vector<int>& hs_nb) {
     ImpState* S = new ImpState();
     ctx->implicit_state = S;

@@ -78,20 +78,11 @@ extern "C" int ccfd_estimate_device_bytes(const ccfd_params* p, const ccfd_mesh*
     double b = 380.0 * N + 40.0 * H + 104.0 * F + 140.0 * B + (1 << 20);
     if (p->precision == CCFD_MIXED && !p->implicit) b += 32.0 * N;
     if (p->source_func) b += 32.0 * N;
-    if (p->implicit) {
-        const double K = (double)(p->n_kdim > 0 ? p->n_kdim : 1);
-        // Krylov bases V (K+1) and Z (K), eight work vectors, D / D^-1 per
-        // cell, off-diagonal blocks per half-side, colouring and sweep lists,
-        // the cluster sweeps' records (two sweeps of at most 4 N + 16384
-        // records of 64 bytes)
-        b += (64.0 * K + 32.0 + 8.0 * 32.0 + 256.0 + 96.0) * N + 144.0 * H + 128.0 * (4.0 * N + 16384.0);
-        // the Jacobian's four columns, as far as the Krylov vectors (idle
-        // meanwhile) do not hold them, and their ghosts
-        const double vec = p->precision == CCFD_MIXED ? 16.0 : 32.0;
-        const double cols = 4.0 * (64.0 * N + 2.0 * vec * (p->eqn == CCFD_NAVIER_STOKES ? N : F));
-        b += 256.0 * B + (cols > 1.8 * K * vec * N ? cols : 0.0);
-    }
-    *bytes = round_up((size_t)(1.2 * b));
+    b *= 1.2;
+    // the implicit arrays are counted one by one: they are most of an implicit
+    // case, and a fifth on top would keep requests out of a budget they fit
+    if (p->implicit) b += 1.03 * (double)ccfd_implicit_bytes(p, m);
+    *bytes = round_up((size_t)b);
     return CCFD_OK;
 }
 
