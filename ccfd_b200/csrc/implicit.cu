@@ -137,7 +137,7 @@ struct ImpState {
     int* color_cells = nullptr;
     int* twin = nullptr;         // [H] half-side of the neighbour that points back
     // LU-SGS level schedules
-    int n_lev_f = 0, n_lev_b = 0, max_level = 0;
+    int n_lev_f = 0, n_lev_b = 0;
     int *lev_f_off = nullptr, *fw_cell = nullptr, *lev_b_off = nullptr, *bw_cell = nullptr;
     int4 *fw_nb = nullptr, *fw_h = nullptr, *bw_nb = nullptr, *bw_h = nullptr;
     bool cluster_ok = false;     // the sweeps fit the cluster kernel
@@ -1573,7 +1573,7 @@ int ccfd_implicit_setup(ccfd_ctx* ctx, const std::vector<int>& hs_off, const std
                     if (n4[q] < 0) continue;
                     if (q >= kClNb) {
                         S->cluster_ok = false;
-                        continue;
+                        return;
                     }
                     r.h[q] = h4[q];
                     const int e = n4[q], we = owner(e);
@@ -1590,6 +1590,7 @@ int ccfd_implicit_setup(ccfd_ctx* ctx, const std::vector<int>& hs_off, const std
                         from.mail[j] = (cta << kClMailBits) | box;
                     } else {
                         S->cluster_ok = false;
+                        return;
                     }
                 }
             }
@@ -1611,13 +1612,11 @@ int ccfd_implicit_setup(ccfd_ctx* ctx, const std::vector<int>& hs_off, const std
         std::vector<int> clo[2];
         std::vector<SweepRec> clr[2];
         sequences(lf, lfc, fwn, fwh, clo[0], clr[0]);
-        sequences(lb, lbc, bwn, bwh, clo[1], clr[1]);
+        if (S->cluster_ok) sequences(lb, lbc, bwn, bwh, clo[1], clr[1]);
         for (int k = 0; k < 2 && S->cluster_ok; ++k)
             if ((st = iupload(ctx, &S->cl_off[k], clo[k])) || (st = iupload(ctx, &S->cl_rec[k], clr[k]))) return st;
         S->n_lev_f = nlf;
         S->n_lev_b = nlb;
-        for (int l = 0; l < nlf; ++l) S->max_level = std::max(S->max_level, lfo[l + 1] - lfo[l]);
-        for (int l = 0; l < nlb; ++l) S->max_level = std::max(S->max_level, lbo[l + 1] - lbo[l]);
         if ((st = iupload(ctx, &S->twin, twin)) || (st = iupload(ctx, &S->color_cells, ccells)) ||
             (st = iupload(ctx, &S->color_off_d, coff)) ||
             (st = iupload(ctx, &S->lev_f_off, lfo)) || (st = iupload(ctx, &S->fw_cell, lfc)) ||
@@ -1657,7 +1656,6 @@ struct ImpSet {
     ImpDev* dev = nullptr;
     std::vector<ImpGroup> groups;
     int n = 0, max_nb = 0, max_col = 0, max_colsize = 0, max_K = 0, max_newton = 0;
-    int max_level = 0;  // widest LU-SGS level (cells) over the members
     bool any_precond = false;
     bool any_plain = false;  // a member without preconditioner
     bool cluster = false;  // LU-SGS by clusters (every preconditioned member fits)
@@ -1775,7 +1773,6 @@ static int set_build(const std::vector<ccfd_ctx*>& members, cudaStream_t stream,
             M->max_col = std::max(M->max_col, ncol);
             for (int c = 0; c < ncol; ++c)
                 M->max_colsize = std::max(M->max_colsize, S->color_off[c + 1] - S->color_off[c]);
-            M->max_level = std::max(M->max_level, S->max_level);
         }
         StageLaunch probe;
         ccfd_fill_stage(ctx, probe);

@@ -111,7 +111,10 @@ inline int4 tile_entry(int inst, int tile, const void* word) {
 
 void launch_stage(const StageLaunch& L, cudaStream_t st);
 void launch_stage_batch(const BatchLaunch& B, cudaStream_t st);
-// limited gradients only (L.grad, and L.grad_out in mixed precision)
+// The gradient kernel alone.  It writes the limited gradients to L.grad_out if
+// that is set, the reconstructed face states (Euler, L.fstate) or the gradients
+// (Navier-Stokes, L.grad), the ghost states at the barycentres and the boundary
+// faces, and, if L.ghost_pface is set, the wall pressures.
 void launch_gradients(const StageLaunch& L, cudaStream_t st);
 // dynamic shared memory of a batched flux launch over tiles of up to max_f faces
 int stage_smem_bytes(int max_f, int fp32);

@@ -72,16 +72,16 @@ struct SmemLimit {
     }
 };
 
-// CTA shapes.  k_grad: 4 / grad_vars threads per cell, at most kGradThreads
-// per CTA.
+// CTA shapes.  k_grad: two threads per cell (kGradVars variables each), at most
+// kGradThreads per CTA.
 // k_flux: at most `threads`, `single` unless the context sets another size.
 // regs / regs_ns (viscous) / grad_regs cap the registers per thread: 76 us per
 // stage (500,000 triangles) at 72 registers in k_grad, 84 at 80, 82 at 64 and
 // 96; viscous flux 48.9 us (200,000 triangles) at 128, 50.0 at 112, 52.3 at 96.
-constexpr int kGradThreads = 128;
+constexpr int kGradThreads = 128, kGradVars = 2;
 template <typename FT> struct StageShape;
-template <> struct StageShape<double> { static constexpr int threads = 384, single = 128, regs = 72, regs_ns = 128, grad_vars = 2, grad_regs = 72; };
-template <> struct StageShape<float> { static constexpr int threads = 256, single = 128, regs = 64, regs_ns = 72, grad_vars = 2, grad_regs = 64; };
+template <> struct StageShape<double> { static constexpr int threads = 384, single = 128, regs = 72, regs_ns = 128, grad_regs = 72; };
+template <> struct StageShape<float> { static constexpr int threads = 256, single = 128, regs = 64, regs_ns = 72, grad_regs = 64; };
 
 __device__ __forceinline__ double stage_time(const Ctrl* ctrl, double tfix, double a_time) {
     return ctrl ? ctrl->t + a_time * ctrl->dt : tfix;
@@ -139,10 +139,7 @@ __device__ __forceinline__ void st32(double4* p, const double4 v) {
 }
 __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
-// VPT consecutive doubles that the kernel may have written itself
-__device__ __forceinline__ void ld_rw(const double* p, double (&v)[1]) {
-    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v[0]) : "l"(p) : "memory");
-}
+// two consecutive doubles that the kernel may have written itself
 __device__ __forceinline__ void ld_rw(const double* p, double (&v)[2]) {
     asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "l"(p) : "memory");
 }
@@ -171,7 +168,7 @@ __device__ __forceinline__ void ld_face(const float4* p, float l[4], float r[4])
                  : "memory");
 }
 
-// shared-memory vector types of the stage kernel: FP64 throughout, or FP32
+// vector types of the stage kernels' arithmetic: FP64 throughout, or FP32
 // reconstruction and face fluxes (mixed precision; state, residual sums and
 // the update stay FP64)
 template <typename T> struct Vec;
@@ -648,15 +645,15 @@ __device__ __forceinline__ void step_end_block(Ctrl* ctrl, const StepParams& sp,
 }
 
 // limited reconstruction of tile t's cells and the ghost states of their
-// boundary sides; 4 / NV consecutive threads treat one cell, thread `part`
-// its variables NV part ... (a fraction of the registers of one thread per
+// boundary sides; two consecutive threads treat one cell, two variables each
+// (a fraction of the registers of one thread per
 // cell, so more warps hide the gathers).  The boundary code runs in loops of
 // its own over the tile's ghosts, before and after the cells: called from the
 // cell loop its registers spilled the loop's.
 template <int LIM, int NS, typename FT>
 __device__ __forceinline__ void grad_body(const StageLaunch& L, const int t) {
     using V4 = typename Vec<FT>::v4;
-    constexpr int NV = StageShape<FT>::grad_vars, G = 4 / NV;
+    constexpr int NV = kGradVars, G = 4 / NV;
     const DevMesh& m = L.mesh;
     const int v0 = NV * (int)(threadIdx.x % G);
     const int d_end = min(m.N, (t + 1) * L.tiles.cells);
@@ -718,8 +715,7 @@ __device__ __forceinline__ void grad_body(const StageLaunch& L, const int t) {
                     for (int v = 0; v < NV; ++v) o[v] = double(f[v]);
                 } else {
                     FT* o = reinterpret_cast<FT*>(L.fstate) + 4 * (size_t)slv[k] + v0;
-                    if constexpr (NV == 2) *reinterpret_cast<typename Vec<FT>::v2*>(o) = typename Vec<FT>::v2{f[0], f[1]};
-                    else *o = f[0];
+                    *reinterpret_cast<typename Vec<FT>::v2*>(o) = typename Vec<FT>::v2{f[0], f[1]};
                 }
             }
         }

@@ -1,5 +1,5 @@
-// Hilbert ordering of cells and construction of the staged tiles of the
-// stage kernels (see tiles.h).
+// Orderings of the cells and construction of the flux kernel's tiles (see
+// tiles.h).
 #include "tiles.h"
 
 #include <algorithm>
