@@ -278,6 +278,11 @@ extern "C" int ccfd_upload_case(ccfd_ctx* ctx, const ccfd_mesh* m, const ccfd_bc
         return CCFD_ERR_ARG;
     for (long g = 0; g < m->n_bc; ++g)
         if (m->bc_index[g] < 0 || m->bc_index[g] >= n_bc) return CCFD_ERR_ARG;
+    // the per-cell records hold three or four sides
+    for (long c = 0; c < m->n_cells; ++c) {
+        const long sides = m->hs_offset[c + 1] - m->hs_offset[c];
+        if (sides < 3 || sides > 4) return CCFD_ERR_ARG;
+    }
     CK(cudaSetDevice(ctx->device));
     free_device(ctx);
     const ccfd_params& p = ctx->params;

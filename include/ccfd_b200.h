@@ -142,7 +142,7 @@ typedef struct ccfd_exact {
  *   faces       0..n_faces-1 in side[] order; the owner is side[f]
  *   half-sides  per cell, CSR in the order of the cell's side list
  *               (elem->firstSide ... nextElemSide), the order of every
- *               per-cell sum of the reference
+ *               per-cell sum of the reference; three or four per cell
  *   ghosts      0..n_bc-1 in BCside[] order; a neighbour index < 0 encodes
  *               ghost b as -1-b
  */
