@@ -184,7 +184,6 @@ __device__ __forceinline__ void block_partial(double v, double* partial) {
 __device__ __forceinline__ double block_total(const double* partial, int nb) {
     __shared__ double sh[kB];
     double v = 0.0;
-#pragma unroll 8
     for (int k = threadIdx.x; k < nb; k += kB) v += partial[k];
     sh[threadIdx.x] = v;
     __syncthreads();
@@ -200,11 +199,11 @@ __device__ __forceinline__ double block_total(const double* partial, int nb) {
 // A dot product in the kernel that needs it: up to kFusedParts partials are
 // summed there by every block, instead of waiting for a launch in between;
 // kb_total leaves the sum of more behind them (what every block reads grows
-// with the square of the mesh).  Milliseconds of an
-// unpreconditioned step of 12 to 16 Krylov iterations, summed in the consumers /
-// by kb_total: 32,768 cells 1.61 / 1.96, 131,072 2.05 / 2.20, 262,144 2.89 /
-// 3.15, 524,288 (2,048 partials) 4.13 / 4.12, 1,048,576 7.08 / 6.75, 2,097,152
-// 13.7 / 12.6, 4,194,304 26.4 / 21.3.
+// with the square of the mesh).  Milliseconds of an unpreconditioned step of 12
+// to 16 Krylov iterations, summed in the consumers / by kb_total: 32,768 cells
+// 1.65 / 1.96, 131,072 2.07 / 2.20, 262,144 2.82 / 3.15, 524,288 (2,048
+// partials) 4.17 / 4.12, 1,048,576 7.18 / 6.70, 2,097,152 14.0 / 12.6, 4,194,304
+// 27.0 / 21.3.
 constexpr int kFusedParts = 2048;
 __device__ __forceinline__ double dot_total(const double* partial, int nb) {
     return nb > kFusedParts ? partial[nb] : block_total(partial, nb);
