@@ -164,8 +164,8 @@ def roofline_bytes_per_residual(n_tri: int, n_quad: int, venk: bool) -> int:
 # k_grad and one k_flux launch) on this workload from one ncu capture, valid
 # only for the kernel sources whose digest is recorded beside it (STAGE_SOURCES); for
 # other sources the line reports no traffic.
-STAGE_TRAFFIC = {"bytes": 83.507e6 + 45.046e6 + 94.817e6 + 27.232e6,
-                 "sha256": "f41ed71d1e66721c"}
+STAGE_TRAFFIC = {"bytes": 77.848e6 + 46.506e6 + 72.240e6 + 30.268e6,
+                 "sha256": "344c3ec9f5918ddb"}
 STAGE_SOURCES = ("ccfd_b200/csrc/stage_impl.cuh", "ccfd_b200/csrc/physics.cuh",
                  "ccfd_b200/csrc/kernels.cuh", "ccfd_b200/csrc/stage_flux.inc",
                  "ccfd_b200/csrc/stage_f05.cu", "ccfd_b200/csrc/gradients.inc",

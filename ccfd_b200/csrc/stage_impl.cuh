@@ -33,7 +33,7 @@
 // warps per SM, ring cells computed twice, half the threads idle in the
 // second pass of each phase.  The split keeps each loop's registers low
 // enough for 28 warps, computes every gradient once and streams the face
-// states: 76, 167 and 13.7 us (62 us with FP32 fluxes), at 0.13 + 0.12 GB of
+// states: 76, 167 and 13.7 us (62 us with FP32 fluxes), at 0.12 + 0.10 GB of
 // DRAM traffic on the 500,000 triangles.  Both kernels are bound by memory
 // latency (the scheduler issues in ~42 % of its cycles) and by chains of
 // correctly rounded FP64 divisions.
@@ -645,11 +645,11 @@ __device__ __forceinline__ void step_end_block(Ctrl* ctrl, const StepParams& sp,
 }
 
 // limited reconstruction of tile t's cells and the ghost states of their
-// boundary sides; two consecutive threads treat one cell, two variables each
-// (a fraction of the registers of one thread per
-// cell, so more warps hide the gathers).  The boundary code runs in loops of
-// its own over the tile's ghosts, before and after the cells: called from the
-// cell loop its registers spilled the loop's.
+// boundary sides; two consecutive threads treat one cell, two variables each (a
+// fraction of the registers of one thread per cell, so more warps hide the
+// gathers).  The boundary code runs in loops of its own over the tile's ghosts,
+// before and after the cells: called from the cell loop its registers spilled
+// the loop's.
 template <int LIM, int NS, typename FT>
 __device__ __forceinline__ void grad_body(const StageLaunch& L, const int t) {
     using V4 = typename Vec<FT>::v4;
